@@ -66,15 +66,16 @@ def listed():
 
 
 def draw(rng):
+    # no attention layer on exactly two rows: its front refuses them (a launch error), as the step and the ragged end of a prompt do
     kind = rng.choice(["gdn", "gdn", "attn", "attn", "attn", "moe", "moe", "moe", "head", "linear", "step", "prefill"])
     tp = rng.choice([1, 2, 4, 8, 8])
-    rows = rng.choice([1, 1, 2, 3, 4, 4, 5, 6, 7, 8, 8])
+    rows = rng.choice([1, 1, 3, 4, 4, 5, 6, 7, 8, 8])
     layers = max(1, tp // 2)
     std = round(math.exp(rng.uniform(math.log(0.02), math.log(2.0))), 4)      # the residual rows grow along the stack
     if kind == "gdn":
-        return {"kind": kind, "tp": tp, "rows": rows, "layers": layers, "position": 16 * rng.randint(0, 8000) + rng.randint(0, 8), "std": std}
+        return {"kind": kind, "tp": tp, "rows": rng.choice([rows, rows, 2]), "layers": layers, "position": 16 * rng.randint(0, 8000) + rng.randint(0, 8), "std": std}
     if kind == "moe":
-        return {"kind": kind, "tp": tp, "rows": rows, "layers": layers, "std": std}
+        return {"kind": kind, "tp": tp, "rows": rng.choice([rows, rows, 2]), "layers": layers, "std": std}
     if kind == "attn":
         keys = int(round(math.exp(rng.uniform(math.log(16), math.log(MAX_KEYS - 16)))))
         return {"kind": kind, "tp": tp, "rows": rows, "keys": keys, "layers": 1 if keys > 65536 else max(1, layers // 2), "std": std}
@@ -84,7 +85,7 @@ def draw(rng):
         return {"kind": kind, "rows": rng.choice([16, 24, 32, 64, 96, 128]), "out": 128 * rng.randint(8, 160), "terms": rng.choice([1, 2, 3])}
     if kind == "step":
         return {"kind": kind, "tp": 8, "rows": rows, "keys": rng.randint(32, 8192), "layers": rng.choice([1, 2, 4])}
-    return {"kind": kind, "tp": 8, "tokens": rng.randint(70, 333), "wide": rng.choice([0, 64, 64, 128]), "layers": 4}
+    return {"kind": kind, "tp": 8, "tokens": rng.choice([n for n in range(70, 333) if n % 8 != 2]), "wide": rng.choice([0, 64, 64, 128]), "layers": 4}
 
 
 # ---- inputs: plain torch, from the seed alone -------------------------------------------------------------------------
@@ -184,9 +185,12 @@ def _prepare_layers(case, seed):
     kind, M = case["kind"], case["rows"]
     spec = ShardSpec(CFG, case["tp"], 0)
     g = _gen(seed)
-    ctxs, blocks, rows, outs = [], [], [], []
-    for _ in range(case["layers"]):
+    ctxs, blocks, outs = [], [], []
+    x = torch.zeros(case["layers"], 8, H, dtype=torch.bfloat16, device=DEV)     # the residual rows of every layer
+    rows = torch.zeros(case["layers"], M, H, dtype=torch.bfloat16, device=DEV)
+    for i in range(case["layers"]):
         c = _context(spec)
+        c.x = x[i]
         if kind == "gdn":
             P = case.get("position", POSITION)
             b = Gdn(c, _gdn_weights(g, spec), state_ring=9)
@@ -202,17 +206,16 @@ def _prepare_layers(case, seed):
             b = Moe(c, _moe_weights(g, spec))
             outs.append([c.x[:M]])
         c.ctl[Ctl.COMMITTED_LEN] = P
-        rows.append(_rows(g, case))
+        rows[i] = _rows(g, case)
         ctxs.append(c)
         blocks.append(b)
-    xs = [c.x[:M] for c in ctxs]
 
     def one_pass():
-        torch._foreach_copy_(xs, rows)      # the layers' input rows (a layer adds its output to them)
+        x[:, :M].copy_(rows)                # the layers' input rows (a layer adds its output to them)
         for b in blocks:
             b.forward(M)
 
-    return {"graph": _captured(one_pass), "outs": outs, "keep": (ctxs, blocks, rows)}
+    return {"graph": _captured(one_pass), "outs": outs, "keep": (ctxs, blocks, x, rows)}
 
 
 def _prepare_head(case, seed):
