@@ -98,8 +98,9 @@ class FullAttn:
                                  c.cp_channel.ref if merge_here else None, cp_site)
             return
         check(
-            lib.nexrt_oproj_allreduce(
-                ptr(c.attn_out), ptr(c.gate), None, ptr(self.w["out_w"]), ptr(self.w["out_s"]), ptr(c.x), cfg.hidden, spec.attn_local, M,
+            lib.nexrt_oproj_rows_allreduce(
+                ptr(c.attn_out), ptr(c.gate), None, ptr(self.w["out_w"]), ptr(self.w["out_s"]), ptr(c.x),
+                ptr(c.oproj_planes), ptr(c.oproj_descale), cfg.hidden, spec.attn_local, M,
                 2 if merge_here else 0, cfg.rms_eps, cfg.head_dim, c.ar_channel.ref, c.next_site(), c.cp_channel.ref if merge_here else None, cp_site,
                 n_cta, st,
             ),

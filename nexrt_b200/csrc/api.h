@@ -73,6 +73,9 @@ int nexrt_attn_decode(const void* q_raw, const void* gate, const void* k_raw, co
 int nexrt_oproj_allreduce(const void* in, const void* z, const void* gnorm_w, const void* w, const void* s, void* x, int H, int K, int M,
                           int mode, float eps, int hd, const NexrtLLChannel* ch, unsigned int site, const NexrtLLChannel* cp,
                           unsigned int cp_site, int n_cta, void* stream);
+int nexrt_oproj_rows_allreduce(const void* in, const void* z, const void* gnorm_w, const void* w, const void* s, void* x, void* planes, void* descale,
+                               int H, int K, int M, int mode, float eps, int hd, const NexrtLLChannel* ch, unsigned int site,
+                               const NexrtLLChannel* cp, unsigned int cp_site, int n_cta, void* stream);   /* planes: e4m3 [3 M][K], descale: [M] scratch */
 
 /* mixture of experts */
 /* w holds E+1 rows; if it is padded with zero rows to rows_pad (a multiple of 16) and `partial`

@@ -457,4 +457,89 @@ __device__ __forceinline__ float mma_bf16_result(const float* tiles, int ksplit,
 // holds 2 rows and two n-tiles hold 4 (5 would fit; 4 keeps the passes even for 8 rows).
 template <int MP> struct MmaShape { static constexpr int TERMS = 3, NT = MP <= 2 ? 1 : 2, TILE = 16 * 8 * NT; };
 
+// Streaming form for several token rows, or for CTAs that walk several 16-row groups: one CTA per group, its warps split
+// the K windows, and a ring of windows per warp is refilled as it is consumed - across the boundary to the CTA's next
+// group too - so the weight stream does not stop while a group is reduced and stored.  NT n-tiles hold the 3 terms of all
+// rows of the step (8 rows: 24 columns), so the weights pass once whatever the row count.  NB: windows in the ring, 9 registers
+// each; a kernel that starts while its predecessor still runs should ask for no more than its K needs (a smaller CTA finds
+// room beside the predecessor's and has its weights in flight earlier).
+template <int NT, int NB>
+struct MmaStream {
+    static constexpr int COLS = 8 * NT;
+    static constexpr int TILE_LD = COLS + 1;             // odd: the reduction reads 16 rows of one column without bank conflicts
+    uint4 ra[NB], rb[NB];
+    float sc[NB];
+    const uint8_t* w;
+    const float* s;
+    int K, nwin, warp, nwarps, g, t;
+
+    __device__ __forceinline__ MmaStream(const uint8_t* w_, const float* s_, int K_, int warp_, int nwarps_)
+        : w(w_), s(s_), K(K_), nwin(K_ / kWin), warp(warp_), nwarps(nwarps_) {
+        const int lane = threadIdx.x & 31;
+        g = lane >> 2; t = lane & 3;
+    }
+    // slot i of step `step` of the group at row0: this warp's window (step * NB + i)
+    __device__ __forceinline__ void fetch(int i, int row0, int step) {
+        const int win = warp + (step * NB + i) * nwarps;
+        if (win < nwin) {
+            const uint8_t* p = w + static_cast<size_t>(row0 + g) * K + win * kWin + t * 16;
+            ra[i] = ld_stream16(p);
+            rb[i] = ld_stream16(p + static_cast<size_t>(8) * K);
+            sc[i] = ld_const_f32(s + (row0 >> 7) * (K >> 7) + (win >> 1));
+        }
+    }
+    __device__ __forceinline__ void preload(int row0) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) fetch(i, row0, 0);
+    }
+    // The group at row0 (its first step is in the ring); afterwards the ring holds the first step of the group at next_row0
+    // (< 0: none).  xq: shared memory e4m3 columns [ncols][ldx], ldx a multiple of 16 (64 bytes over a multiple of 128:
+    // neighbouring columns start 16 banks apart, so the 16-byte reads of two of them do not conflict).
+    __device__ __forceinline__ void group(int row0, int next_row0, const uint8_t* xq, int ldx, int ncols, float (&d)[NT][4]) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+        const int steps = (nwin + NB * nwarps - 1) / (NB * nwarps);
+        for (int st = 0; st < steps; ++st) {
+            const bool more = st + 1 < steps;
+            const int frow = more ? row0 : next_row0, fstep = more ? st + 1 : 0;
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const int win = warp + (st * NB + i) * nwarps;
+                if (win < nwin) {                        // uniform across the warp
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        const int col = nt * 8 + g;
+                        uint4 xb = make_uint4(0u, 0u, 0u, 0u);
+                        if (col < ncols) xb = *reinterpret_cast<const uint4*>(xq + static_cast<size_t>(col) * ldx + win * kWin + t * 16);
+                        float c[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_e4m3_16x8x32(c, ra[i].x, rb[i].x, ra[i].y, rb[i].y, xb.x, xb.y);
+                        mma_e4m3_16x8x32(c, ra[i].z, rb[i].z, ra[i].w, rb[i].w, xb.z, xb.w);
+                        d[nt][0] = fmaf(c[0], sc[i], d[nt][0]); d[nt][1] = fmaf(c[1], sc[i], d[nt][1]);
+                        d[nt][2] = fmaf(c[2], sc[i], d[nt][2]); d[nt][3] = fmaf(c[3], sc[i], d[nt][3]);
+                    }
+                }
+                if (frow >= 0) fetch(i, frow, fstep);
+            }
+        }
+    }
+    // This warp's partial of the group: tiles[warp][16][TILE_LD].
+    __device__ __forceinline__ void store(float* tiles, const float (&d)[NT][4]) const {
+        float* tile = tiles + warp * 16 * TILE_LD;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            tile[g * TILE_LD + nt * 8 + 2 * t] = d[nt][0]; tile[g * TILE_LD + nt * 8 + 2 * t + 1] = d[nt][1];
+            tile[(g + 8) * TILE_LD + nt * 8 + 2 * t] = d[nt][2]; tile[(g + 8) * TILE_LD + nt * 8 + 2 * t + 1] = d[nt][3];
+        }
+    }
+    // Product of weight row `row` of the group with token row m: the warps' partials, then the terms, in the order of mma_result.
+    static __device__ __forceinline__ float result(const float* tiles, int warps, int row, int m, float descale) {
+        float v = 0.f;
+        for (int k = 0; k < warps; ++k) {
+            const float* p = tiles + (k * 16 + row) * TILE_LD + 3 * m;
+            v = fmaf(p[2], kTermInv * kTermInv, fmaf(p[1], kTermInv, v + p[0]));
+        }
+        return v * descale;
+    }
+};
+
 }  // namespace nexrt

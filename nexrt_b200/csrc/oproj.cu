@@ -38,6 +38,8 @@ struct OProjArgs {
     unsigned int site;
     LLChannel cp;           // mode 2: partial inbox of the context-parallel group
     unsigned int cp_site;
+    const uint8_t* planes;  // staged form: e4m3 terms [3 M][K] and the row scales [M]
+    const float* descale;
 };
 
 template <int MB>
@@ -120,91 +122,177 @@ __global__ void __launch_bounds__(512, 1) oproj_allreduce_kernel(OProjArgs a) {
     allreduce_residual(a.ch, a.site, res, a.M, row0, nrows, a.H, a.x, a.overwrite == 0, a.partial_out);
 }
 
-// Tensor-core form: one CTA per 16 output rows, the 8 warps split K (see mma_gemv.cuh); the CTA
-// that computed the rows reduces them across the ranks and updates the residual.
-template <int MP>
-__global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a) {
-    constexpr int TERMS = MmaShape<MP>::TERMS, NT = MmaShape<MP>::NT, TILE = MmaShape<MP>::TILE, NB = 8;
+// Four consecutive values k .. k + 3 of input row m (mode 0: plain; mode 1: gated RMSNorm of a 128-wide head, which one warp
+// holds; mode 2: context-parallel merge of the group's partials).
+template <int MODE>
+__device__ __forceinline__ float4 oproj_input4(const OProjArgs& a, int m, int k, const float4& o, const float4& zz, const float4& gw, const LLCall& cpcall) {
+    if (MODE == 0) return o;
+    if (MODE == 1) {
+        const float inv = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / 128.f + a.eps);
+        return make_float4(gw.x * o.x * inv * silu_f(zz.x), gw.y * o.y * inv * silu_f(zz.y), gw.z * o.z * inv * silu_f(zz.z), gw.w * o.w * inv * silu_f(zz.w));
+    }
+    const int hd = a.hd, heads = a.K / hd;
+    const float gate[4] = {zz.x, zz.y, zz.z, zz.w};
+    float r[4];
+    for (int i = 0; i < 4; ++i) {
+        const int lh = (k + i) / hd, d = (k + i) % hd;
+        const unsigned int base = (static_cast<unsigned int>(m) * heads + lh) * (hd + 1);
+        float lse[kMaxWorld], ctx[kMaxWorld], mx = -INFINITY;
+        for (int sr = 0; sr < a.cp.world; ++sr) {
+            unsigned int pl, pc;
+            ll_wait(a.cp, cpcall, sr, base + hd, &pl, kStatusCpTimeout);
+            ll_wait(a.cp, cpcall, sr, base + d, &pc, kStatusCpTimeout);
+            lse[sr] = __uint_as_float(pl);
+            ctx[sr] = __uint_as_float(pc);
+            mx = fmaxf(mx, lse[sr]);
+        }
+        float num = 0.f, den = 0.f;
+        for (int sr = 0; sr < a.cp.world; ++sr) {
+            const float wgt = lse[sr] == -INFINITY ? 0.f : exp2f(lse[sr] - mx);
+            num = fmaf(wgt, ctx[sr], num);
+            den += wgt;
+        }
+        r[i] = (den > 0.f ? num / den : 0.f) * sigmoid_f(gate[i]);
+    }
+    return make_float4(r[0], r[1], r[2], r[3]);
+}
+
+constexpr int kOprojWarps = 8;
+constexpr int kOprojPad = 64;      // bytes behind each activation column (see MmaStream::group)
+// Shared memory of the kernel below without and with the fp32 copy of the input rows.
+template <int NT> constexpr size_t oproj_smem(int M, int K) {
+    return static_cast<size_t>(M) * 3 * (K + kOprojPad) + sizeof(float) * 2 * kOprojWarps * 16 * MmaStream<NT, 8>::TILE_LD;
+}
+
+// Tensor-core form: the 8 warps of a CTA split K and walk the CTA's groups of 16 output rows (see MmaStream); the CTA that
+// computed the rows reduces them across the ranks and updates the residual.  All rows of the step go through in one pass.
+//
+// What bounds it is the chain input -> split -> product -> store, not the weights (4 MB per rank at the 8-way shard).  One
+// warp computes a whole 128-wide block of one row and the rows' largest magnitudes meet in shared memory, so however many
+// rows there are the input takes two barriers (scale known, terms written); staged four rows at a time with a reduction of
+// its own per row, eight rows took two passes over the weights and about twenty barriers.  The values wait for the scale in
+// shared memory (`keep`), or are computed a second time where that memory would cost the SM its second CTA.
+//
+// MODE 3: the terms and row scales were made by a kernel in front (oproj_stage_split_kernel) and are only copied in.  Made
+// here, they are made again by every CTA, and that - about 150 instructions per block and warp - is what several rows then
+// cost.  One B200, 8-way shard (K = 1024), cost of the projection in the layer at 8 rows: 15.7 us staged four rows at a time,
+// 12 us made here, 2.5 + 3.9 us with the kernel in front.
+template <int NT, int MODE, int NB>
+__global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a, int keep) {
+    using Stream = MmaStream<NT, NB>;
+    constexpr int U = MODE == 2 ? 1 : 2;                                  // blocks of a warp in flight (next to the weight ring: 128 registers)
     extern __shared__ __align__(16) float smem[];
-    __shared__ float red[32];
-    __shared__ float descale[MP];
+    __shared__ unsigned int s_max[kMaxRows];                             // bits of the largest magnitude of each row
     TraceCta tr;
     tr.begin(kTrOproj);
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int row0 = blockIdx.x * kRowsPerGroup, nwin = a.K / kWin;
-    const int KS = min(nwarps, nwin);                                   // warps that share the K range
-    float* xs = smem;                                                   // [MP][K]
-    float* tiles = xs + static_cast<size_t>(MP) * a.K;                  // [KS][16][8]
-    float* res = tiles + 8 * TILE;                                       // [kMaxRows][16]
-    uint8_t* xq = reinterpret_cast<uint8_t*>(res + kMaxRows * kRowsPerGroup);   // [MP*TERMS][K]
-    const MmaPlain src{a.w, a.s, a.K};
-    MmaWarp<NB, MmaPlain> mw(row0, warp, KS, warp < KS ? nwin : 0);
-    mw.preload(src);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = a.K / 128, ldx = a.K + kOprojPad, items = a.M * nb;
+    float* tiles = smem;                                                  // [2][8][16][TILE_LD]
+    constexpr int kTiles = kOprojWarps * 16 * Stream::TILE_LD;
+    uint8_t* xq = reinterpret_cast<uint8_t*>(tiles + 2 * kTiles);         // [3 M][ldx]
+    float* xs = reinterpret_cast<float*>(xq + static_cast<size_t>(a.M) * 3 * ldx);   // [M][K] (keep)
+    if (MODE != 3 && threadIdx.x < kMaxRows) s_max[threadIdx.x] = 0u;
+    Stream mw(a.w, a.s, a.K, warp, kOprojWarps);
+    int row0 = blockIdx.x * kRowsPerGroup;
+    mw.preload(row0);
+    __syncthreads();
     pdl_wait();
     tr.mark(1);
-    LLCall cpcall{0u, 0u};
-    if (a.mode == 2) cpcall = ll_begin(a.cp, a.cp_site);
-    for (int m0 = 0; m0 < a.M; m0 += MP) {
-        const int mb = min(MP, a.M - m0);
-        if (m0) { __syncthreads(); mw.next_pass(); }
-        if (a.mode == 0) {
-            for (int idx = threadIdx.x * 4; idx < mb * a.K; idx += blockDim.x * 4)
-                *reinterpret_cast<float4*>(xs + idx) = *reinterpret_cast<const float4*>(a.in + static_cast<size_t>(m0) * a.K + idx);
-        } else if (a.mode == 1) {
-            const int heads = a.K / 128;
-            const float4 gw = *reinterpret_cast<const float4*>(a.gnorm_w + lane * 4);
-            for (int v = warp; v < mb * heads; v += nwarps) {
-                const int m = v / heads, h = v % heads;
-                const size_t base = static_cast<size_t>(m0 + m) * a.K + h * 128 + lane * 4;
-                const float4 o = *reinterpret_cast<const float4*>(a.in + base);
-                const float4 zz = *reinterpret_cast<const float4*>(a.z + base);
-                const float inv = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / 128.f + a.eps);
-                float4 r;
-                r.x = gw.x * o.x * inv * silu_f(zz.x);
-                r.y = gw.y * o.y * inv * silu_f(zz.y);
-                r.z = gw.z * o.z * inv * silu_f(zz.z);
-                r.w = gw.w * o.w * inv * silu_f(zz.w);
-                *reinterpret_cast<float4*>(xs + m * a.K + h * 128 + lane * 4) = r;
-            }
-        } else {
-            const int hd = a.hd, heads = a.K / hd;
-            for (int idx = threadIdx.x; idx < mb * a.K; idx += blockDim.x) {
-                const int m = idx / a.K, k = idx % a.K, lh = k / hd, d = k % hd;
-                const unsigned int base = (static_cast<unsigned int>(m0 + m) * heads + lh) * (hd + 1);
-                float lse[kMaxWorld], ctx[kMaxWorld], mx = -INFINITY;
-                for (int sr = 0; sr < a.cp.world; ++sr) {
-                    unsigned int pl, pc;
-                    ll_wait(a.cp, cpcall, sr, base + hd, &pl, kStatusCpTimeout);
-                    ll_wait(a.cp, cpcall, sr, base + d, &pc, kStatusCpTimeout);
-                    lse[sr] = __uint_as_float(pl);
-                    ctx[sr] = __uint_as_float(pc);
-                    mx = fmaxf(mx, lse[sr]);
-                }
-                float num = 0.f, den = 0.f;
-                for (int sr = 0; sr < a.cp.world; ++sr) {
-                    const float wgt = lse[sr] == -INFINITY ? 0.f : exp2f(lse[sr] - mx);
-                    num = fmaf(wgt, ctx[sr], num);
-                    den += wgt;
-                }
-                const float gt = a.z[static_cast<size_t>(m0 + m) * a.K + k];
-                xs[m * a.K + k] = (den > 0.f ? num / den : 0.f) * sigmoid_f(gt);
-            }
+    LLCall call{0u, 0u}, cpcall{0u, 0u};
+    if (a.ch.world > 1) call = ll_begin(a.ch, a.site);
+    if (MODE == 2) cpcall = ll_begin(a.cp, a.cp_site);
+    // thread (r, m) owns output row r of a group for token row m
+    const int er = threadIdx.x % kRowsPerGroup, em = threadIdx.x / kRowsPerGroup;
+    const bool owner = em < a.M;
+    float descale = 0.f;
+    if constexpr (MODE == 3) {
+        const int pieces = a.K / 16;
+        for (int i = threadIdx.x; i < a.M * 3 * pieces; i += blockDim.x) {
+            const int col = i / pieces, c = i % pieces;
+            const unsigned int dst = static_cast<unsigned int>(__cvta_generic_to_shared(xq + static_cast<size_t>(col) * ldx + c * 16));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(a.planes + static_cast<size_t>(i) * 16) : "memory");
         }
-        __syncthreads();
-        act_split<TERMS>(xq, xs, mb, a.K, red, descale);
-        float d[NT][4];
-        mw.template run<NT>(src, xq, a.K, mb * TERMS, d);
-        if (warp < KS) mw.template store<NT>(tiles + warp * TILE, d);
-        __syncthreads();
-        if (threadIdx.x < kRowsPerGroup * mb) {
-            const int rl = threadIdx.x % kRowsPerGroup, m = threadIdx.x / kRowsPerGroup;
-            res[(m0 + m) * kRowsPerGroup + rl] = mma_result<TERMS, NT>(tiles, KS, rl, m, descale[m]);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (owner) descale = a.descale[em];
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+    float4 gw = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (MODE == 1) gw = *reinterpret_cast<const float4*>(a.gnorm_w + lane * 4);
+    // input block v of this warp (row v / nb): what four values of it are made from
+    auto request = [&](int v, float4& o, float4& zz) {
+        const size_t at = static_cast<size_t>(v) * 128 + lane * 4;
+        o = zz = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v < items) {
+            if (MODE != 2) o = *reinterpret_cast<const float4*>(a.in + at);
+            if (MODE != 0) zz = *reinterpret_cast<const float4*>(a.z + at);
+        }
+    };
+    for (int v0 = warp; v0 < items; v0 += U * kOprojWarps) {
+        float4 o[U], zz[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) request(v0 + u * kOprojWarps, o[u], zz[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int v = v0 + u * kOprojWarps;
+            if (v < items) {                                              // uniform across the warp
+                const float4 x4 = oproj_input4<MODE>(a, v / nb, (v % nb) * 128 + lane * 4, o[u], zz[u], gw, cpcall);
+                const float mx = warp_max(fmaxf(fmaxf(fabsf(x4.x), fabsf(x4.y)), fmaxf(fabsf(x4.z), fabsf(x4.w))));
+                if (lane == 0) atomicMax(&s_max[v / nb], __float_as_uint(mx));
+                if (keep) *reinterpret_cast<float4*>(xs + static_cast<size_t>(v) * 128 + lane * 4) = x4;
+            }
         }
     }
     __syncthreads();
-    tr.mark(2);
-    allreduce_residual(a.ch, a.site, res, a.M, row0, kRowsPerGroup, a.H, a.x, a.overwrite == 0, a.partial_out);
+    // biased exponent of the power of two that brings the row's largest magnitude into [128, 256); 2^8 for a row without one,
+    // as act_split has it; capped so that the factor and its inverse are normal numbers
+    auto up_exp = [&](int m) {
+        const float mx = __uint_as_float(s_max[m]);
+        return mx > 0.f && mx < 3.0e38f ? min(261 - static_cast<int>(s_max[m] >> 23), 253) : 135;
+    };
+    for (int v = warp; v < items; v += kOprojWarps) {
+        const int m = v / nb, b = v % nb;
+        float4 x4;
+        if (keep) {
+            x4 = *reinterpret_cast<const float4*>(xs + static_cast<size_t>(v) * 128 + lane * 4);   // this thread's own values
+        } else {
+            float4 o, zz;
+            request(v, o, zz);
+            x4 = oproj_input4<MODE>(a, m, b * 128 + lane * 4, o, zz, gw, cpcall);
+        }
+        const float up = __uint_as_float(static_cast<unsigned int>(up_exp(m)) << 23);
+        float r[4] = {x4.x * up, x4.y * up, x4.z * up, x4.w * up};
+        uint32_t out[3];
+        split4<3>(r, out);
+#pragma unroll
+        for (int term = 0; term < 3; ++term) *reinterpret_cast<uint32_t*>(xq + static_cast<size_t>(m * 3 + term) * ldx + b * 128 + lane * 4) = out[term];
+    }
+    if (owner) descale = __uint_as_float(static_cast<unsigned int>(254 - up_exp(em)) << 23);
+    }
+    __syncthreads();
+    for (int buf = 0; row0 < a.H; buf ^= 1) {
+        const int next = row0 + static_cast<int>(gridDim.x) * kRowsPerGroup;
+        const size_t o = static_cast<size_t>(em) * a.H + row0 + er;
+        __nv_bfloat16 res = __ushort_as_bfloat16(0);        // requested before the product and kept as read: a conversion here would wait for it
+        if (owner && !a.overwrite) res = a.x[o];
+        float d[NT][4];
+        mw.group(row0, next < a.H ? next : -1, xq, ldx, 3 * a.M, d);
+        // two tile buffers: the barrier of the next group separates this group's readers from the writers after it
+        float* tl = tiles + buf * kTiles;
+        mw.store(tl, d);
+        __syncthreads();
+        tr.mark(2);
+        if (owner) {
+            const float v = Stream::result(tl, kOprojWarps, er, em, descale);
+            if (a.partial_out != nullptr) {
+                a.partial_out[o] = v;
+            } else {
+                const float sum = ll_allreduce_f32(a.ch, call, static_cast<unsigned int>(o), v);
+                a.x[o] = __float2bfloat16_rn(a.overwrite ? sum : __bfloat162float(res) + sum);
+            }
+        }
+        row0 = next;
+    }
     tr.mark(3);
 }
 
@@ -212,7 +300,7 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
 // (mode 0 plain copy, 1 GDN gated RMSNorm with z, 2 context-parallel merge of the group's partials) and writes it as
 // three e4m3 planes [3M][K] plus a power-of-two scale per row - the B operand of the tcgen05 GEMM that follows
 // (nexrt_tc_oproj_allreduce in tc_moe.cu), which also does the all-reduce and the residual.
-__global__ void __launch_bounds__(256) oproj_stage_split_kernel(OProjArgs a, uint8_t* planes, float* descale_out) {
+__global__ void __launch_bounds__(1024) oproj_stage_split_kernel(OProjArgs a, uint8_t* planes, float* descale_out) {
     extern __shared__ __align__(16) float xs[];          // [K]
     __shared__ float red[32];
     __shared__ float ds[1];
@@ -276,8 +364,36 @@ extern "C" int nexrt_oproj_stage_split(const void* in, const void* z, const void
     a.in = static_cast<const float*>(in); a.z = static_cast<const float*>(z); a.gnorm_w = static_cast<const float*>(gnorm_w);
     a.K = K; a.M = M; a.mode = mode; a.hd = hd; a.eps = eps;
     if (cp) { a.cp = *cp; a.cp_site = cp_site; }
-    return launch(oproj_stage_split_kernel, dim3(M), dim3(256), sizeof(float) * K, static_cast<cudaStream_t>(stream), a, static_cast<uint8_t*>(planes),
+    return launch(oproj_stage_split_kernel, dim3(M), dim3(max(128, min(1024, K / 4))), sizeof(float) * K, static_cast<cudaStream_t>(stream), a, static_cast<uint8_t*>(planes),
                   static_cast<float*>(descale));
+}
+
+// Launches the tensor-core form (mode 3: staged terms); -1 when its shared memory does not fit.  The columns of all rows stay
+// in shared memory: an unsharded K of 8192 with eight rows just fits, anything wider takes the CUDA-core kernel.
+static int launch_oproj_mma(const OProjArgs& a, int mode, cudaStream_t st) {
+    const int nt = (3 * a.M + 7) / 8, groups = a.H / kRowsPerGroup;
+    const size_t base = nt == 1 ? oproj_smem<1>(a.M, a.K) : (nt == 2 ? oproj_smem<2>(a.M, a.K) : oproj_smem<3>(a.M, a.K)), half = 112 * 1024, all = 226 * 1024;
+    if (base > all) return -1;
+    const size_t kept = base + sizeof(float) * a.M * a.K;
+    const int keep = mode != 3 && kept <= (base <= half ? half : all) ? 1 : 0;
+    const int resident = sm_count() * (base <= half ? 2 : 1);
+    const int rounds = (groups + resident - 1) / resident;
+    const dim3 g((groups + rounds - 1) / rounds), b(256);                // as few CTAs as the rounds need: each stages the input once
+    auto go = [&](auto kernel) { return launch(kernel, g, b, keep ? kept : base, st, a, keep); };
+    // windows of one warp per group: the ring holds two, four or (wide K) eight of them, six beside 24 columns
+    const int wpw = (a.K / kWin + kOprojWarps - 1) / kOprojWarps;
+    if (nt == 1) {
+        auto by_mode = [&](auto plain, auto gated, auto merge, auto staged) { return mode == 0 ? go(plain) : (mode == 1 ? go(gated) : (mode == 2 ? go(merge) : go(staged))); };
+        if (wpw <= 2) return by_mode(oproj_allreduce_mma_kernel<1, 0, 2>, oproj_allreduce_mma_kernel<1, 1, 2>, oproj_allreduce_mma_kernel<1, 2, 2>, oproj_allreduce_mma_kernel<1, 3, 2>);
+        if (wpw <= 4) return by_mode(oproj_allreduce_mma_kernel<1, 0, 4>, oproj_allreduce_mma_kernel<1, 1, 4>, oproj_allreduce_mma_kernel<1, 2, 4>, oproj_allreduce_mma_kernel<1, 3, 4>);
+        return by_mode(oproj_allreduce_mma_kernel<1, 0, 8>, oproj_allreduce_mma_kernel<1, 1, 8>, oproj_allreduce_mma_kernel<1, 2, 8>, oproj_allreduce_mma_kernel<1, 3, 8>);
+    }
+    if (nt == 2) {
+        if (mode != 3) return mode == 0 ? go(oproj_allreduce_mma_kernel<2, 0, 4>) : (mode == 1 ? go(oproj_allreduce_mma_kernel<2, 1, 4>) : go(oproj_allreduce_mma_kernel<2, 2, 4>));
+        return wpw <= 2 ? go(oproj_allreduce_mma_kernel<2, 3, 2>) : (wpw <= 4 ? go(oproj_allreduce_mma_kernel<2, 3, 4>) : go(oproj_allreduce_mma_kernel<2, 3, 8>));
+    }
+    if (mode != 3) return mode == 0 ? go(oproj_allreduce_mma_kernel<3, 0, 4>) : (mode == 1 ? go(oproj_allreduce_mma_kernel<3, 1, 4>) : go(oproj_allreduce_mma_kernel<3, 2, 4>));
+    return wpw <= 2 ? go(oproj_allreduce_mma_kernel<3, 3, 2>) : (wpw <= 4 ? go(oproj_allreduce_mma_kernel<3, 3, 4>) : go(oproj_allreduce_mma_kernel<3, 3, 6>));
 }
 
 extern "C" int nexrt_oproj_allreduce(const void* in, const void* z, const void* gnorm_w, const void* w, const void* s, void* x, int H, int K,
@@ -295,15 +411,9 @@ extern "C" int nexrt_oproj_allreduce(const void* in, const void* z, const void* 
     a.partial_out = partial_out_buffer();
     if (cp) { a.cp = *cp; a.cp_site = cp_site; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int mp = M == 1 ? 1 : (M == 2 ? 2 : 4), terms = 3;
-    const size_t smem_mma = sizeof(float) * (static_cast<size_t>(mp) * K + 8 * 256 + kMaxRows * 16) + static_cast<size_t>(mp) * terms * K;
-    // wide K with several rows (an unsharded out-projection at tensor-parallel 1) does not fit the tensor-core
-    // kernel's staging buffers: those shapes take the CUDA-core kernel
-    if ((gemv_mode() & 2) && H % 16 == 0 && K % 64 == 0 && smem_mma <= 200 * 1024) {
-        dim3 g(H / 16), b(256);
-        if (mp == 1) return launch(oproj_allreduce_mma_kernel<1>, g, b, smem_mma, st, a);
-        if (mp == 2) return launch(oproj_allreduce_mma_kernel<2>, g, b, smem_mma, st, a);
-        return launch(oproj_allreduce_mma_kernel<4>, g, b, smem_mma, st, a);
+    if ((gemv_mode() & 2) && H % 16 == 0) {
+        const int e = launch_oproj_mma(a, mode, st);
+        if (e >= 0) return e;
     }
     const int mb = M == 1 ? 1 : 4;
     const int max_rows = (H + n_cta - 1) / n_cta;
@@ -312,4 +422,23 @@ extern "C" int nexrt_oproj_allreduce(const void* in, const void* z, const void* 
     dim3 g(n_cta), b(gemv_threads());
     if (mb == 1) return launch(oproj_allreduce_kernel<1>, g, b, smem, st, a);
     return launch(oproj_allreduce_kernel<4>, g, b, smem, st, a);
+}
+
+// The same with scratch for the input's terms (planes: e4m3 [3 M][K], descale: fp32 [M]): made once by a kernel of their own
+// instead of by every CTA.  The line: several rows always gain (see above); one row gains where K is wide - an unsharded
+// 8192 takes 4.0 + 8.1 us against 14.6, 4096 a layer of 29.1 us against 30.8, 2048 no difference, and at 1024 the second
+// node costs more than the eight blocks that every CTA computes.
+extern "C" int nexrt_oproj_rows_allreduce(const void* in, const void* z, const void* gnorm_w, const void* w, const void* s, void* x, void* planes, void* descale,
+                                          int H, int K, int M, int mode, float eps, int hd, const NexrtLLChannel* ch, unsigned int site,
+                                          const NexrtLLChannel* cp, unsigned int cp_site, int n_cta, void* stream) {
+    const bool staged = M >= 1 && (M >= 2 || K >= 4096) && M <= kMaxRows && (gemv_mode() & 2) && H % 16 == 0 && K % 128 == 0 && ch != nullptr && planes != nullptr && descale != nullptr &&
+                        (ch->world <= 1 || ch->slots >= static_cast<unsigned int>(kMaxRows) * H) && oproj_smem<3>(M, K) <= 226 * 1024;
+    if (!staged) return nexrt_oproj_allreduce(in, z, gnorm_w, w, s, x, H, K, M, mode, eps, hd, ch, site, cp, cp_site, n_cta, stream);
+    if (const int e = nexrt_oproj_stage_split(in, z, gnorm_w, planes, descale, K, M, mode, eps, hd, cp, cp_site, stream)) return e;
+    OProjArgs a{};
+    a.w = static_cast<const uint8_t*>(w); a.s = static_cast<const float*>(s); a.x = static_cast<__nv_bfloat16*>(x);
+    a.H = H; a.K = K; a.M = M; a.mode = 3; a.hd = hd; a.overwrite = (mode & 4) ? 1 : 0; a.eps = eps; a.ch = *ch; a.site = site;
+    a.partial_out = partial_out_buffer();
+    a.planes = static_cast<const uint8_t*>(planes); a.descale = static_cast<const float*>(descale);
+    return launch_oproj_mma(a, 3, static_cast<cudaStream_t>(stream));
 }

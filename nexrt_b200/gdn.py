@@ -89,8 +89,9 @@ class Gdn:
             wide.oproj_allreduce(c, c.gdn_out, c.gdn_z, w["gnorm_w"], w["out_w"], w["out_s"], spec.gdn_local, M, 1, 128, None, 0)
             return
         check(
-            lib.nexrt_oproj_allreduce(
-                ptr(c.gdn_out), ptr(c.gdn_z), ptr(w["gnorm_w"]), ptr(w["out_w"]), ptr(w["out_s"]), ptr(c.x), cfg.hidden, spec.gdn_local,
+            lib.nexrt_oproj_rows_allreduce(
+                ptr(c.gdn_out), ptr(c.gdn_z), ptr(w["gnorm_w"]), ptr(w["out_w"]), ptr(w["out_s"]), ptr(c.x),
+                ptr(c.oproj_planes), ptr(c.oproj_descale), cfg.hidden, spec.gdn_local,
                 M, 1, cfg.rms_eps, 128, c.ar_channel.ref, c.next_site(), None, 0, n_cta, st,
             ),
             "gdn_oproj_allreduce",

@@ -58,6 +58,7 @@ _PROTOTYPES = {
     "nexrt_attn_decode_merges_cp": [ci],
     "nexrt_attn_decode": [vp] * 14 + [ci] * 8 + [cf, ci, ci, ci, ci, ci, ci, CH, cu, vp],
     "nexrt_oproj_allreduce": [vp] * 6 + [ci] * 4 + [cf, ci, CH, cu, CH, cu, ci, vp],
+    "nexrt_oproj_rows_allreduce": [vp] * 8 + [ci] * 4 + [cf, ci, CH, cu, CH, cu, ci, vp],
     "nexrt_moe_router": [vp] * 8 + [ci] * 5 + [cf, ci, vp, vp],
     "nexrt_moe_l1": [vp] * 6 + [ci] * 4 + [cf, ci, ci, vp],
     "nexrt_moe_router_partial": [vp] * 4 + [ci] * 5 + [cf, vp, vp],

@@ -66,7 +66,7 @@ def main() -> None:
         print(f"rows={a.rows} ctx={a.ctx} layers={cfg.n_layers}: {full:.1f} us/step")
         if a.leave_one_out:
             real = eng.ctx.lib
-            for name in ("nexrt_gdn_front", "nexrt_gdn_core", "nexrt_attn_front", "nexrt_attn_decode", "nexrt_oproj_allreduce", "nexrt_moe_router",
+            for name in ("nexrt_gdn_front", "nexrt_gdn_core", "nexrt_attn_front", "nexrt_attn_decode", "nexrt_oproj_rows_allreduce", "nexrt_moe_router",
                          "nexrt_moe_l1", "nexrt_moe_l2_allreduce", "nexrt_lmhead_sample", "nexrt_rows_norm_split", "nexrt_tc_rows_gemm",
                          "nexrt_gdn_front_tail", "nexrt_tc_router_logits", "nexrt_moe_router_topk", "nexrt_tc_moe_l1", "nexrt_tc_moe_l2_allreduce",
                          "nexrt_lmhead_sample_from_logits"):
