@@ -174,12 +174,12 @@ int nexrt_tc_moe_l2_allreduce(const void* gu, const void* ids, const void* wts, 
                               void* stream);
 
 // ---- wide (multi-row) projections on tcgen05 ---------------------------------------------------------------------
-int nexrt_rows_norm_split(const void* x, const void* gamma, void* planes, void* xn, int H, int M, float eps, void* stream);
-int nexrt_tc_rows_gemm(const void* w, const void* w_s, const void* planes, void* out, const void* zero_ids, int R, int K, int M, int ksplit, int* status,
-                       void* stream);   /* out: [ksplit][M][R] partial planes */
-int nexrt_gdn_front_tail(const void* pre, const void* xn, const void* ba_w, const void* conv_w, const void* a_log, const void* dt_bias, const void* ctl,
-                         void* conv_ring, void* qkv, void* z, void* beta, void* g, int H, int R, int C, int nv, int M, int conv_ring_len, int ksplit,
-                         void* stream);
+   /* out: [ksplit][M][R] partial planes */
+int nexrt_gdn_front_rows(const void* x, const void* in_ln, const void* front_w, const void* front_s, const void* ba_w, const void* conv_w, const void* a_log,
+                         const void* dt_bias, const void* ctl, void* conv_ring, void* qkv, void* z, void* beta, void* g, void* cols, int H, int R, int C,
+                         int nv, int M, int conv_ring_len, float eps, void* stream);   /* 2..8 rows; cols: f16 [2 M][H] scratch */
+int nexrt_attn_front_rows(const void* x, const void* in_ln, const void* w, const void* s, const void* ctl, void* q_raw, void* gate, void* k_raw,
+                          void* v_cache, void* cols, int H, int hd, int nq, int ngate, int kvh, int M, int cache_len, float eps, void* stream);
 
 int nexrt_tc_router_logits(const void* x, const void* gamma, const void* w, void* planes, void* partial, const void* zero_ids, int rows, int rows_pad, int K,
                            int M, int ksplit, float eps, void* planes_e4m3, int* status, void* stream);   /* partial: [ksplit][M][rows_pad] */

@@ -151,6 +151,59 @@ __global__ void __launch_bounds__(256, 2) attn_front_mma_kernel(AttnFrontArgs a)
     tr.mark(3);
 }
 
+// Front of several rows: the rows' f16 columns come from a kernel in front, the weights stream once for all of them (see
+// gdn_front_rows_kernel, the same product with another tail).  One B200, 8-way shard, the layer's front at 8 rows: 2.5 + 6.6 + 9.2 us
+// as a tcgen05 GEMM split over K with a tail kernel -> 2.7 + 6.5 us.
+__global__ void __launch_bounds__(256) rows_norm_f16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, __half* cols, int H, float eps) {
+    extern __shared__ __align__(16) float xs[];          // [H]
+    __shared__ float red[32];
+    TraceCta tr;
+    tr.begin(kTrHelper);
+    pdl_launch_dependents();
+    RowNorm<4> norm;
+    norm.preload_gamma(gamma, H);
+    pdl_wait();
+    tr.mark(1);
+    const size_t m = blockIdx.x;
+    row_norm_f16(norm, cols + m * 2 * H, xs, x + m * H, H, eps, red);
+    tr.mark(3);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(512, 1) attn_front_rows_kernel(AttnFrontArgs a, const uint8_t* __restrict__ cols) {
+    using Stream = MmaStreamF16<NT, 8>;
+    extern __shared__ __align__(16) float smem[];
+    TraceCta tr;
+    tr.begin(kTrAttnFront);
+    pdl_launch_dependents();
+    const int team = threadIdx.x >> 8, teams = blockDim.x >> 8, tid = threadIdx.x & 255, ldx = 2 * a.H + kF16Pad, R = (a.nq + a.ngate + 2 * a.kvh) * a.hd;
+    float* tiles = smem + team * kStreamWarps * 16 * Stream::TILE_LD;
+    uint8_t* xq = reinterpret_cast<uint8_t*>(smem + teams * kStreamWarps * 16 * Stream::TILE_LD);
+    Stream mw(a.w, a.s, a.H, tid >> 5);
+    int row0 = (static_cast<int>(blockIdx.x) * teams + team) * kRowsPerGroup;
+    const int stride = static_cast<int>(gridDim.x) * teams * kRowsPerGroup;
+    if (row0 < R) mw.preload(row0);
+    pdl_wait();
+    tr.mark(1);
+    const int C0 = a.ctl[kCtlCommittedLen];
+    const bool interleaved = a.ngate == a.nq;
+    stage_columns(xq, ldx, cols, 2 * a.M, 2 * a.H);
+    __syncthreads();
+    auto team_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory"); };
+    const int er = tid % kRowsPerGroup, em = tid / kRowsPerGroup;
+    while (row0 < R) {
+        const int next = row0 + stride;
+        float d[NT][4];
+        mw.group(row0, next < R ? next : -1, xq, ldx, 2 * a.M, d);
+        mw.store(tiles, d);
+        team_sync();
+        if (em < a.M) attn_front_row(a, row0 + er, em, Stream::result(tiles, er, em, kSplitDescale), C0, interleaved);
+        if (next < R) team_sync();                                    // the tile is read before the next group writes it
+        row0 = next;
+    }
+    tr.mark(3);
+}
+
 struct AttnDecodeArgs {
     const float* q_raw;       // [M][nq][hd]
     const float* gate;        // [M][ngate][hd]
@@ -178,8 +231,8 @@ struct AttnDecodeArgs {
     unsigned long long* events;   // optional timing ring: split 0 records phases 0..5, the combining CTA 6..9
 };
 
-// Tail of the wide front (multi-row steps): the projections of all rows come from the tcgen05 rows GEMM as K-split
-// partial planes pre[ks][M][R]; one thread per weight row adds them in order and scatters the row's M values.
+// Tail of a prefill chunk's front: the projections of all its rows come from the GEMM (as K-split partial planes pre[ks][M][R]);
+// one thread per weight row adds them in order and scatters the row's M values.
 __global__ void __launch_bounds__(256) attn_front_tail_kernel(AttnFrontArgs a, const float* __restrict__ pre, int R, int ksplit) {
     TraceCta tr;
     tr.begin(kTrHelper);
@@ -942,6 +995,24 @@ extern "C" int nexrt_attn_front(const void* x, const void* in_ln, const void* w,
     const size_t smem = sizeof(float) * (static_cast<size_t>(mb + 1) * H + gemv_part_floats((R + n_cta - 1) / n_cta, mb, gemv_geom(H / 16, gemv_threads())));
     if (M == 1) return launch(attn_front_kernel<1>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
     return launch(attn_front_kernel<4>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
+}
+
+// The front of 2..8 rows (cols: f16 [2 M][H] scratch).  cudaErrorNotSupported, with nothing launched, for shapes outside this
+// form and with the tensor-core fronts switched off: the caller then takes nexrt_attn_front.
+extern "C" int nexrt_attn_front_rows(const void* x, const void* in_ln, const void* w, const void* s, const void* ctl, void* q_raw, void* gate, void* k_raw,
+                                     void* v_cache, void* cols, int H, int hd, int nq, int ngate, int kvh, int M, int cache_len, float eps, void* stream) {
+    if (M < 1 || M > kMaxRows || H % 256 || (hd != 128 && hd != 256)) return cudaErrorInvalidValue;
+    if (!(gemv_mode() & 1) || H > 4096) return cudaErrorNotSupported;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (const int e = launch(rows_norm_f16_kernel, dim3(M), dim3(256), sizeof(float) * H, st, static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(in_ln),
+                             static_cast<__half*>(cols), H, eps)) return e;
+    AttnFrontArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(in_ln), static_cast<const uint8_t*>(w),
+                    static_cast<const float*>(s), static_cast<const int*>(ctl), static_cast<float*>(q_raw), static_cast<float*>(gate),
+                    static_cast<float*>(k_raw), static_cast<__nv_bfloat16*>(v_cache), H, hd, nq, ngate, kvh, M, cache_len, eps};
+    const FrontRows f(M, H, (nq + ngate + 2 * kvh) * hd / kRowsPerGroup);
+    const uint8_t* cp = static_cast<const uint8_t*>(cols);
+    return f.nt == 1 ? launch(attn_front_rows_kernel<1>, dim3(f.grid), dim3(256 * f.teams), f.smem, st, a, cp)
+                     : launch(attn_front_rows_kernel<2>, dim3(f.grid), dim3(256 * f.teams), f.smem, st, a, cp);
 }
 
 // Optional timing ring (16 x u64 device memory) filled by the decode kernel of kv head 0; null switches it off.

@@ -247,83 +247,127 @@ __global__ void __launch_bounds__(256, 2) gdn_front_mma_kernel(GdnFrontArgs a) {
     tr.mark(3);
 }
 
-// Tail of the wide front (multi-row steps): the q|k|v|z projections of all rows were produced by the tcgen05 rows
-// GEMM into pre[M][R]; this kernel applies the per-channel conv ring + SiLU / the z store (one thread per weight
-// row, all token rows in registers), and extra CTAs project the bf16 b/a rows from the fp32 normalised rows xn.
-__global__ void __launch_bounds__(256) gdn_front_tail_kernel(GdnFrontArgs a, const float* __restrict__ pre, const float* __restrict__ xn, int row_ctas,
-                                                             int ksplit) {
+// ---- front of several rows: two kernels ----------------------------------------------------------------------------------
+// First the rows: one CTA per (token row, eight b/a rows) normalises the row, and the CTAs of the first b/a group write its
+// f16 columns ([2 M][H]).  The b/a weights of the CTA are in registers before the dependency wait.
+constexpr int kBaRows = 8;
+__global__ void __launch_bounds__(256) gdn_rows_norm_ba_kernel(GdnFrontArgs a, __half* cols) {
+    extern __shared__ __align__(16) float xs[];          // [H]
+    __shared__ float red[32];
+    __shared__ float part[8][kBaRows];
     TraceCta tr;
     tr.begin(kTrHelper);
     pdl_launch_dependents();
+    const int m = blockIdx.x, b0 = blockIdx.y * kBaRows, nb = min(kBaRows, 2 * a.nv - b0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NCH = 4;
+    RowNorm<NCH> norm;
+    norm.preload_gamma(a.in_ln, a.H);
+    uint2 w[kBaRows][NCH];
+#pragma unroll
+    for (int r = 0; r < kBaRows; ++r)
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            const int k = (c * 256 + threadIdx.x) * 4;
+            w[r][c] = r < nb && k < a.H ? *reinterpret_cast<const uint2*>(a.ba_w + static_cast<size_t>(b0 + r) * a.H + k) : make_uint2(0u, 0u);
+        }
     pdl_wait();
     tr.mark(1);
-    if (static_cast<int>(blockIdx.x) < row_ctas) {
-        const int row = blockIdx.x * blockDim.x + threadIdx.x;
-        if (row >= a.R) return;
-        // Every load of the thread is requested before the first use: the three history taps (positions C0 - 3 .. C0 - 1
-        // of the ring, independent of this step's projections), the conv weights, and up to 8 x 8 K-split partials.  In
-        // program order (sum, store the ring, read the ring back) the same work is four dependent trips to L2.
+    row_norm_f16(norm, blockIdx.y == 0 ? cols + static_cast<size_t>(m) * 2 * a.H : nullptr, xs, a.x + static_cast<size_t>(m) * a.H, a.H, a.eps, red);
+    float acc[kBaRows];
+#pragma unroll
+    for (int r = 0; r < kBaRows; ++r) acc[r] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+        const int k = (c * 256 + threadIdx.x) * 4;
+        if (k < a.H) {
+            const float4 v = *reinterpret_cast<const float4*>(xs + k);
+#pragma unroll
+            for (int r = 0; r < kBaRows; ++r)
+                acc[r] = fmaf(__uint_as_float(w[r][c].x << 16), v.x, fmaf(__uint_as_float(w[r][c].x & 0xffff0000u), v.y,
+                         fmaf(__uint_as_float(w[r][c].y << 16), v.z, fmaf(__uint_as_float(w[r][c].y & 0xffff0000u), v.w, acc[r]))));
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kBaRows; ++r) {
+        const float t = warp_sum(acc[r]);
+        if (lane == 0) part[warp][r] = t;
+    }
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < nb) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += part[k][threadIdx.x];        // fixed order over the warps
+        gdn_ba_row(a, b0 + threadIdx.x, v, m);
+    }
+    tr.mark(3);
+}
+
+// Then the projection: the weights stream once for all rows (MmaStreamF16) against the columns in shared memory, and the team
+// of warps that holds a 16-row group's products applies the conv ring, SiLU and the z store itself.
+//
+// It is bound by the weight stream and its conversion on wide shards, by the chain columns -> product -> store on narrow ones.
+// Before, the projections ran as a tcgen05 GEMM split over K whose fp32 partial planes a third kernel added (or, below four
+// rows, as the one-row kernel twice).  One B200, 8-way shard, the layer's front at 8 rows: 2.9 + 6.9 + 5.5 us -> 4.7 + 6.6 us; an
+// unsharded layer of 8 rows 124 -> 71 us, of 3 rows 139 -> 56 us (the out-projection included).
+template <int NT>
+__global__ void __launch_bounds__(512, 1) gdn_front_rows_kernel(GdnFrontArgs a, const uint8_t* __restrict__ cols) {
+    using Stream = MmaStreamF16<NT, 8>;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float s_taps[2][kMaxRows + 3][kRowsPerGroup];          // positions C0 - 3 .. C0 + M - 1 of a group's channels
+    TraceCta tr;
+    tr.begin(kTrGdnFront);
+    pdl_launch_dependents();
+    const int team = threadIdx.x >> 8, teams = blockDim.x >> 8, tid = threadIdx.x & 255, ldx = 2 * a.H + kF16Pad, ring = a.conv_ring_len;
+    float* tiles = smem + team * kStreamWarps * 16 * Stream::TILE_LD;
+    uint8_t* xq = reinterpret_cast<uint8_t*>(smem + teams * kStreamWarps * 16 * Stream::TILE_LD);
+    float (*taps)[kRowsPerGroup] = s_taps[team];
+    Stream mw(a.front_w, a.front_s, a.H, tid >> 5);
+    int row0 = (static_cast<int>(blockIdx.x) * teams + team) * kRowsPerGroup;
+    const int stride = static_cast<int>(gridDim.x) * teams * kRowsPerGroup;
+    if (row0 < a.R) mw.preload(row0);
+    pdl_wait();
+    tr.mark(1);
+    const int C0 = a.ctl[kCtlCommittedLen];
+    stage_columns(xq, ldx, cols, 2 * a.M, 2 * a.H);
+    __syncthreads();
+    tr.mark(4);
+    auto team_sync = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory"); };
+    const int er = tid % kRowsPerGroup, em = tid / kRowsPerGroup;     // thread (r, m): row r of the group, token row m
+    while (row0 < a.R) {
+        const int next = row0 + stride, row = row0 + er;
         const bool conv = row < a.C;
-        const int C0 = a.ctl[kCtlCommittedLen], ring = a.conv_ring_len;
-        float hist[3] = {0.f, 0.f, 0.f};
+        // history and conv weights are requested before the product
+        float hist = 0.f;
         float4 cw = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (conv) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) hist[j] = __ldcg(a.conv_ring + static_cast<size_t>((C0 - 3 + j + ring) % ring) * a.C + row);
-            cw = *reinterpret_cast<const float4*>(a.conv_w + static_cast<size_t>(row) * 4);
-        }
-        constexpr int kMaxSplit = 8;
-        float part[kMaxRows][kMaxSplit];
-#pragma unroll
-        for (int m = 0; m < kMaxRows; ++m)
-#pragma unroll
-            for (int ks = 0; ks < kMaxSplit; ++ks)
-                part[m][ks] = (m < a.M && ks < ksplit) ? __ldcg(pre + (static_cast<size_t>(ks) * a.M + m) * a.R + row) : 0.f;
-        float p[kMaxRows];
-#pragma unroll
-        for (int m = 0; m < kMaxRows; ++m) {
-            p[m] = 0.f;
-#pragma unroll
-            for (int ks = 0; ks < kMaxSplit; ++ks) p[m] += part[m][ks];      // K-split partials, fixed order (absent ones are zero)
-        }
-        if (!conv) {
-#pragma unroll
-            for (int m = 0; m < kMaxRows; ++m)
-                if (m < a.M) a.z[static_cast<size_t>(m) * (a.R - a.C) + (row - a.C)] = p[m];
-        } else {
-            // window of the causal conv: positions C0 - 3 .. C0 + M - 1
-#pragma unroll
-            for (int m = 0; m < kMaxRows; ++m) {
-                if (m < a.M) {
-                    const float h0 = m >= 3 ? p[m - 3 < 0 ? 0 : m - 3] : hist[m], h1 = m >= 2 ? p[m - 2 < 0 ? 0 : m - 2] : hist[m + 1],
-                                h2 = m >= 1 ? p[m - 1 < 0 ? 0 : m - 1] : hist[m + 2 > 2 ? 2 : m + 2];
-                    const float v = fmaf(cw.x, h0, fmaf(cw.y, h1, fmaf(cw.z, h2, cw.w * p[m])));
-                    a.conv_ring[static_cast<size_t>((C0 + m) % ring) * a.C + row] = p[m];
-                    a.qkv[static_cast<size_t>(m) * a.C + row] = silu_f(v);
+        if (em < 3 && conv) hist = __ldcg(a.conv_ring + static_cast<size_t>((C0 - 3 + em + ring) % ring) * a.C + row);
+        if (em < a.M && conv) cw = *reinterpret_cast<const float4*>(a.conv_w + static_cast<size_t>(row) * 4);
+        float d[NT][4];
+        mw.group(row0, next < a.R ? next : -1, xq, ldx, 2 * a.M, d);
+        mw.store(tiles, d);
+        team_sync();
+        tr.mark(2);
+        if (em < kMaxRows) {                                          // the team's first four warps, whole
+            float p = 0.f;
+            if (em < a.M) {
+                p = Stream::result(tiles, er, em, kSplitDescale);
+                if (conv) {
+                    a.conv_ring[static_cast<size_t>((C0 + em) % ring) * a.C + row] = p;
+                    taps[em + 3][er] = p;
+                } else {
+                    a.z[static_cast<size_t>(em) * (a.R - a.C) + (row - a.C)] = p;
                 }
             }
+            if (em < 3) taps[em][er] = hist;
+            asm volatile("bar.sync %0, 128;" ::"r"(3 + team) : "memory");
+            if (em < a.M && conv) {
+                const float v = fmaf(cw.x, taps[em][er], fmaf(cw.y, taps[em + 1][er], fmaf(cw.z, taps[em + 2][er], cw.w * p)));
+                a.qkv[static_cast<size_t>(em) * a.C + row] = silu_f(v);
+            }
         }
-        tr.mark(3);
-        return;
+        if (next < a.R) team_sync();                                  // the tile and the taps are read before the next group writes them
+        row0 = next;
     }
-    // one warp per (b/a row, token row)
-    const int lane = threadIdx.x & 31;
-    const int item = (blockIdx.x - row_ctas) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= 2 * a.nv * a.M) return;
-    const int row = item / a.M, m = item % a.M;
-    const __nv_bfloat16* w = a.ba_w + static_cast<size_t>(row) * a.H;
-    const float* xr = xn + static_cast<size_t>(m) * a.H;
-    float acc = 0.f;
-#pragma unroll 4
-    for (int k = lane * 8; k < a.H; k += 256) {      // unrolled so that the loads of four steps are in flight together
-        float wf[8];
-        unpack8_bf16(*reinterpret_cast<const uint4*>(w + k), wf);
-        const float4 x0 = *reinterpret_cast<const float4*>(xr + k), x1 = *reinterpret_cast<const float4*>(xr + k + 4);
-        acc = fmaf(wf[0], x0.x, fmaf(wf[1], x0.y, fmaf(wf[2], x0.z, fmaf(wf[3], x0.w, acc))));
-        acc = fmaf(wf[4], x1.x, fmaf(wf[5], x1.y, fmaf(wf[6], x1.z, fmaf(wf[7], x1.w, acc))));
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) gdn_ba_row(a, row, acc, m);
     tr.mark(3);
 }
 
@@ -459,18 +503,24 @@ extern "C" int nexrt_gdn_front(const void* x, const void* in_ln, const void* fro
     return launch(gdn_front_kernel<4>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
 }
 
-// Tail of the wide front: pre [M][R] fp32 projections, xn [M][H] fp32 normalised rows (see gdn_front_tail_kernel).
-extern "C" int nexrt_gdn_front_tail(const void* pre, const void* xn, const void* ba_w, const void* conv_w, const void* a_log, const void* dt_bias,
-                                    const void* ctl, void* conv_ring, void* qkv, void* z, void* beta, void* g, int H, int R, int C, int nv, int M,
-                                    int conv_ring_len, int ksplit, void* stream) {
+// The front of 2..8 rows (cols: f16 [2 M][H] scratch).  cudaErrorNotSupported, with nothing launched, for shapes outside
+// this form and with the tensor-core fronts switched off: the caller then takes nexrt_gdn_front.
+extern "C" int nexrt_gdn_front_rows(const void* x, const void* in_ln, const void* front_w, const void* front_s, const void* ba_w, const void* conv_w,
+                                    const void* a_log, const void* dt_bias, const void* ctl, void* conv_ring, void* qkv, void* z, void* beta, void* g,
+                                    void* cols, int H, int R, int C, int nv, int M, int conv_ring_len, float eps, void* stream) {
     if (M < 1 || M > kMaxRows || H % 256 || conv_ring_len < M + 3) return cudaErrorInvalidValue;
-    GdnFrontArgs a{nullptr, nullptr, nullptr, nullptr, static_cast<const __nv_bfloat16*>(ba_w), static_cast<const float*>(conv_w),
+    if (!(gemv_mode() & 1) || R % 16 || H > 4096) return cudaErrorNotSupported;
+    GdnFrontArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(in_ln), static_cast<const uint8_t*>(front_w),
+                   static_cast<const float*>(front_s), static_cast<const __nv_bfloat16*>(ba_w), static_cast<const float*>(conv_w),
                    static_cast<const float*>(a_log), static_cast<const float*>(dt_bias), static_cast<const int*>(ctl),
                    static_cast<float*>(conv_ring), static_cast<float*>(qkv), static_cast<float*>(z), static_cast<float*>(beta),
-                   static_cast<float*>(g), H, R, C, nv, M, conv_ring_len, 0.f, 0, nullptr};
-    const int row_ctas = (R + 255) / 256, ba_ctas = (2 * nv * M + 7) / 8;
-    return launch(gdn_front_tail_kernel, dim3(row_ctas + ba_ctas), dim3(256), 0, static_cast<cudaStream_t>(stream), a, static_cast<const float*>(pre),
-                  static_cast<const float*>(xn), row_ctas, ksplit);
+                   static_cast<float*>(g), H, R, C, nv, M, conv_ring_len, eps, 0, nullptr};
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (const int e = launch(gdn_rows_norm_ba_kernel, dim3(M, (2 * nv + kBaRows - 1) / kBaRows), dim3(256), sizeof(float) * H, st, a, static_cast<__half*>(cols))) return e;
+    const FrontRows f(M, H, R / kRowsPerGroup);
+    const uint8_t* cp = static_cast<const uint8_t*>(cols);
+    return f.nt == 1 ? launch(gdn_front_rows_kernel<1>, dim3(f.grid), dim3(256 * f.teams), f.smem, st, a, cp)
+                     : launch(gdn_front_rows_kernel<2>, dim3(f.grid), dim3(256 * f.teams), f.smem, st, a, cp);
 }
 
 extern "C" int nexrt_gdn_core(const void* qkv, const void* beta, const void* g, const void* ctl, void* state_ring, void* out, int nqk, int nv,

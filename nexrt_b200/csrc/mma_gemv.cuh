@@ -542,4 +542,180 @@ struct MmaStream {
     }
 };
 
+constexpr int kStreamWarps = 8;
+constexpr int kStreamPad = 64;      // bytes behind each activation column (see MmaStream::group)
+
+// Asynchronous copy of the step's activation columns ([ncols][col_bytes] in global memory, col_bytes a multiple of 16) into
+// shared memory columns ldx bytes apart; complete for this thread on return.  One warp per column, and every CTA starts at another place: all CTAs read
+// the same lines, and in the same order they would queue at one L2 slice after the other.
+__device__ __forceinline__ void stage_columns(uint8_t* xq, int ldx, const uint8_t* planes, int ncols, int col_bytes) {
+    const int pieces = col_bytes / 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int rot = static_cast<int>(blockIdx.x * 37u % static_cast<unsigned int>(pieces));
+    for (int j = warp; j < ncols; j += nw) {
+        const int col = (j + static_cast<int>(blockIdx.x)) % ncols;
+        const uint8_t* src = planes + static_cast<size_t>(col) * col_bytes;
+        const unsigned int dst = static_cast<unsigned int>(__cvta_generic_to_shared(xq + static_cast<size_t>(col) * ldx));
+        for (int c0 = lane; c0 < pieces; c0 += 32) {
+            const int c = c0 + rot < pieces ? c0 + rot : c0 + rot - pieces;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * c), "l"(src + 16 * c) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// ---- the same stream with f16 columns --------------------------------------------------------------------------------------
+// mma.sync on e4m3 operands converts both of them to f16 first, for every n-tile again: 8 rows (24 columns, 3 n-tiles) cost 173
+// cycles per window and scheduler (B200, two warps each).  Here the weights are converted once per window and the
+// columns are f16 already: a row's value (the sum of its three terms, at most 2^-22 of it lost) is hi + lo, so 8 rows are
+// 16 columns, 2 n-tiles, 117 cycles.  Column m holds hi of row m / 2 (m even) or lo.
+constexpr int kF16Pad = 16;         // bytes behind each f16 column: the 16-byte reads of neighbouring columns do not conflict
+
+__device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void e4m3x4_to_f16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(w));
+}
+
+// Four scaled values of a row as f16 hi and lo (packed pairs), after the rounding of the three-term split.
+__device__ __forceinline__ void split4_f16(float (&r)[4], uint2& hi, uint2& lo) {
+    uint32_t t[3];
+    split4<3>(r, t);
+    float v[4], f[4];
+    e4m3x4_to_float4(t[2], v);
+#pragma unroll
+    for (int term = 1; term >= 0; --term) {
+        e4m3x4_to_float4(t[term], f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = fmaf(v[i], kTermInv, f[i]);
+    }
+    const __half2 h0 = __floats2half2_rn(v[0], v[1]), h1 = __floats2half2_rn(v[2], v[3]);
+    const float2 g0 = __half22float2(h0), g1 = __half22float2(h1);
+    const __half2 l0 = __floats2half2_rn(v[0] - g0.x, v[1] - g0.y), l1 = __floats2half2_rn(v[2] - g1.x, v[3] - g1.y);
+    hi = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+    lo = make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
+}
+
+// rmsnorm(x) * gamma of one row into shared memory (xs [K], fp32) and, when `cols` is given, as f16 columns cols[0..K) (hi) and
+// cols[K..2K) (lo).  256 threads, K <= 4096; the thread that reads a value in xs later need not be the one that wrote it.
+__device__ __forceinline__ void row_norm_f16(RowNorm<4>& norm, __half* cols, float* xs, const __nv_bfloat16* x, int K, float eps, float* red) {
+    norm.run<3>(nullptr, xs, x, 1, K, eps, red);
+    if (cols == nullptr) return;
+    for (int k = threadIdx.x * 4; k < K; k += blockDim.x * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(xs + k);
+        float r[4] = {v.x * kSplitScale, v.y * kSplitScale, v.z * kSplitScale, v.w * kSplitScale};
+        uint2 hi, lo;
+        split4_f16(r, hi, lo);
+        *reinterpret_cast<uint2*>(cols + k) = hi;
+        *reinterpret_cast<uint2*>(cols + K + k) = lo;
+    }
+}
+
+template <int NT, int NB>
+struct MmaStreamF16 {
+    static constexpr int COLS = 8 * NT;
+    static constexpr int TILE_LD = COLS + 1;
+    uint4 ra[NB], rb[NB];
+    float sc[NB];
+    const uint8_t* w;
+    const float* s;
+    int K, nwin, warp, g, t;
+
+    __device__ __forceinline__ MmaStreamF16(const uint8_t* w_, const float* s_, int K_, int warp_) : w(w_), s(s_), K(K_), nwin(K_ / kWin), warp(warp_) {
+        const int lane = threadIdx.x & 31;
+        g = lane >> 2; t = lane & 3;
+    }
+    __device__ __forceinline__ void fetch(int i, int row0, int step) {
+        const int win = warp + (step * NB + i) * kStreamWarps;
+        if (win < nwin) {
+            const uint8_t* p = w + static_cast<size_t>(row0 + g) * K + win * kWin + t * 16;
+            ra[i] = ld_stream16(p);
+            rb[i] = ld_stream16(p + static_cast<size_t>(8) * K);
+            sc[i] = ld_const_f32(s + (row0 >> 7) * (K >> 7) + (win >> 1));
+        }
+    }
+    __device__ __forceinline__ void preload(int row0) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) fetch(i, row0, 0);
+    }
+    // As MmaStream::group; xq: shared memory f16 columns [ncols], ldx = 2 K + kF16Pad bytes apart.
+    __device__ __forceinline__ void group(int row0, int next_row0, const uint8_t* xq, int ldx, int ncols, float (&d)[NT][4]) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+        const int steps = (nwin + NB * kStreamWarps - 1) / (NB * kStreamWarps);
+        for (int st = 0; st < steps; ++st) {
+            const bool more = st + 1 < steps;
+            const int frow = more ? row0 : next_row0, fstep = more ? st + 1 : 0;
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const int win = warp + (st * NB + i) * kStreamWarps;
+                if (win < nwin) {                        // uniform across the warp
+                    float c[NT][4];
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {        // half of the lane's 16 weight bytes and 16 column values
+                        uint32_t a[2][4];
+                        e4m3x4_to_f16x4(h ? ra[i].z : ra[i].x, a[0][0], a[0][2]);
+                        e4m3x4_to_f16x4(h ? rb[i].z : rb[i].x, a[0][1], a[0][3]);
+                        e4m3x4_to_f16x4(h ? ra[i].w : ra[i].y, a[1][0], a[1][2]);
+                        e4m3x4_to_f16x4(h ? rb[i].w : rb[i].y, a[1][1], a[1][3]);
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) {
+                            const int col = nt * 8 + g;
+                            uint4 xb = make_uint4(0u, 0u, 0u, 0u);
+                            if (col < ncols) xb = *reinterpret_cast<const uint4*>(xq + static_cast<size_t>(col) * ldx + win * (2 * kWin) + t * 32 + h * 16);
+                            mma_f16_16x8x16(c[nt], a[0][0], a[0][1], a[0][2], a[0][3], xb.x, xb.y);
+                            mma_f16_16x8x16(c[nt], a[1][0], a[1][1], a[1][2], a[1][3], xb.z, xb.w);
+                        }
+                    }
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        d[nt][0] = fmaf(c[nt][0], sc[i], d[nt][0]); d[nt][1] = fmaf(c[nt][1], sc[i], d[nt][1]);
+                        d[nt][2] = fmaf(c[nt][2], sc[i], d[nt][2]); d[nt][3] = fmaf(c[nt][3], sc[i], d[nt][3]);
+                    }
+                }
+                if (frow >= 0) fetch(i, frow, fstep);
+            }
+        }
+    }
+    __device__ __forceinline__ void store(float* tiles, const float (&d)[NT][4]) const {
+        float* tile = tiles + warp * 16 * TILE_LD;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            tile[g * TILE_LD + nt * 8 + 2 * t] = d[nt][0]; tile[g * TILE_LD + nt * 8 + 2 * t + 1] = d[nt][1];
+            tile[(g + 8) * TILE_LD + nt * 8 + 2 * t] = d[nt][2]; tile[(g + 8) * TILE_LD + nt * 8 + 2 * t + 1] = d[nt][3];
+        }
+    }
+    // Product of weight row `row` of the group with token row m, in warp order.
+    static __device__ __forceinline__ float result(const float* tiles, int row, int m, float descale) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < kStreamWarps; ++k) {
+            const float* p = tiles + (k * 16 + row) * TILE_LD + 2 * m;
+            v += p[0] + p[1];
+        }
+        return v * descale;
+    }
+};
+
+// Shape of a front of several rows: teams of eight warps, each with a 16-row group of its own, share the columns in shared
+// memory.  Up to four rows' columns (66 KB at H = 4096) are staged by each of two CTAs per SM; more are staged once, by one CTA
+// of two teams (six rows, unsharded gated-delta-net layer: 92 us with two CTAs, 64 us with one, the out-projection's two teams included).
+struct FrontRows {
+    int nt, teams, grid;
+    size_t smem;
+    FrontRows(int M, int K, int groups) {
+        nt = (2 * M + 7) / 8;
+        const size_t cols = static_cast<size_t>(2 * M) * (2 * K + kF16Pad), tile = sizeof(float) * kStreamWarps * 16 * (8 * nt + 1);
+        teams = cols > 72 * 1024 ? 2 : 1;
+        smem = cols + teams * tile;
+        const int resident = sm_count() * (teams == 2 ? 1 : 2), items = (groups + teams - 1) / teams, rounds = (items + resident - 1) / resident;
+        grid = (items + rounds - 1) / rounds;
+    }
+};
+
 }  // namespace nexrt

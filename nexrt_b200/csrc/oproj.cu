@@ -157,11 +157,9 @@ __device__ __forceinline__ float4 oproj_input4(const OProjArgs& a, int m, int k,
     return make_float4(r[0], r[1], r[2], r[3]);
 }
 
-constexpr int kOprojWarps = 8;
-constexpr int kOprojPad = 64;      // bytes behind each activation column (see MmaStream::group)
 // Shared memory of the kernel below without and with the fp32 copy of the input rows.
 template <int NT> constexpr size_t oproj_smem(int M, int K) {
-    return static_cast<size_t>(M) * 3 * (K + kOprojPad) + sizeof(float) * 2 * kOprojWarps * 16 * MmaStream<NT, 8>::TILE_LD;
+    return static_cast<size_t>(M) * 3 * (K + kStreamPad) + sizeof(float) * 2 * kStreamWarps * 16 * MmaStream<NT, 8>::TILE_LD;
 }
 
 // Tensor-core form: the 8 warps of a CTA split K and walk the CTA's groups of 16 output rows (see MmaStream); the CTA that
@@ -178,7 +176,7 @@ template <int NT> constexpr size_t oproj_smem(int M, int K) {
 // cost.  One B200, 8-way shard (K = 1024), cost of the projection in the layer at 8 rows: 15.7 us staged four rows at a time,
 // 12 us made here, 2.5 + 3.9 us with the kernel in front.
 template <int NT, int MODE, int NB>
-__global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a, int keep) {
+__global__ void __launch_bounds__(MODE == 3 ? 512 : 256, MODE == 3 ? 1 : 2) oproj_allreduce_mma_kernel(OProjArgs a, int keep) {
     using Stream = MmaStream<NT, NB>;
     constexpr int U = MODE == 2 ? 1 : 2;                                  // blocks of a warp in flight (next to the weight ring: 128 registers)
     extern __shared__ __align__(16) float smem[];
@@ -186,16 +184,19 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
     TraceCta tr;
     tr.begin(kTrOproj);
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nb = a.K / 128, ldx = a.K + kOprojPad, items = a.M * nb;
+    // MODE 3: one team of eight warps, or two that share the columns (and then have one tile buffer each)
+    const int team = MODE == 3 ? threadIdx.x >> 8 : 0, teams = MODE == 3 ? blockDim.x >> 8 : 1, tid = threadIdx.x & 255;
+    const int lane = threadIdx.x & 31, warp = tid >> 5;
+    const int nb = a.K / 128, ldx = a.K + kStreamPad, items = a.M * nb;
     float* tiles = smem;                                                  // [2][8][16][TILE_LD]
-    constexpr int kTiles = kOprojWarps * 16 * Stream::TILE_LD;
+    constexpr int kTiles = kStreamWarps * 16 * Stream::TILE_LD;
     uint8_t* xq = reinterpret_cast<uint8_t*>(tiles + 2 * kTiles);         // [3 M][ldx]
     float* xs = reinterpret_cast<float*>(xq + static_cast<size_t>(a.M) * 3 * ldx);   // [M][K] (keep)
     if (MODE != 3 && threadIdx.x < kMaxRows) s_max[threadIdx.x] = 0u;
-    Stream mw(a.w, a.s, a.K, warp, kOprojWarps);
-    int row0 = blockIdx.x * kRowsPerGroup;
-    mw.preload(row0);
+    Stream mw(a.w, a.s, a.K, warp, kStreamWarps);
+    int row0 = (static_cast<int>(blockIdx.x) * teams + team) * kRowsPerGroup;
+    const int stride = static_cast<int>(gridDim.x) * teams * kRowsPerGroup;
+    if (row0 < a.H) mw.preload(row0);
     __syncthreads();
     pdl_wait();
     tr.mark(1);
@@ -203,19 +204,12 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
     if (a.ch.world > 1) call = ll_begin(a.ch, a.site);
     if (MODE == 2) cpcall = ll_begin(a.cp, a.cp_site);
     // thread (r, m) owns output row r of a group for token row m
-    const int er = threadIdx.x % kRowsPerGroup, em = threadIdx.x / kRowsPerGroup;
+    const int er = tid % kRowsPerGroup, em = tid / kRowsPerGroup;
     const bool owner = em < a.M;
     float descale = 0.f;
     if constexpr (MODE == 3) {
-        const int pieces = a.K / 16;
-        for (int i = threadIdx.x; i < a.M * 3 * pieces; i += blockDim.x) {
-            const int col = i / pieces, c = i % pieces;
-            const unsigned int dst = static_cast<unsigned int>(__cvta_generic_to_shared(xq + static_cast<size_t>(col) * ldx + c * 16));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(a.planes + static_cast<size_t>(i) * 16) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
         if (owner) descale = a.descale[em];
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        stage_columns(xq, ldx, a.planes, 3 * a.M, a.K);
     } else {
     float4 gw = make_float4(1.f, 1.f, 1.f, 1.f);
     if (MODE == 1) gw = *reinterpret_cast<const float4*>(a.gnorm_w + lane * 4);
@@ -228,13 +222,13 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
             if (MODE != 0) zz = *reinterpret_cast<const float4*>(a.z + at);
         }
     };
-    for (int v0 = warp; v0 < items; v0 += U * kOprojWarps) {
+    for (int v0 = warp; v0 < items; v0 += U * kStreamWarps) {
         float4 o[U], zz[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) request(v0 + u * kOprojWarps, o[u], zz[u]);
+        for (int u = 0; u < U; ++u) request(v0 + u * kStreamWarps, o[u], zz[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int v = v0 + u * kOprojWarps;
+            const int v = v0 + u * kStreamWarps;
             if (v < items) {                                              // uniform across the warp
                 const float4 x4 = oproj_input4<MODE>(a, v / nb, (v % nb) * 128 + lane * 4, o[u], zz[u], gw, cpcall);
                 const float mx = warp_max(fmaxf(fmaxf(fabsf(x4.x), fabsf(x4.y)), fmaxf(fabsf(x4.z), fabsf(x4.w))));
@@ -250,7 +244,7 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
         const float mx = __uint_as_float(s_max[m]);
         return mx > 0.f && mx < 3.0e38f ? min(261 - static_cast<int>(s_max[m] >> 23), 253) : 135;
     };
-    for (int v = warp; v < items; v += kOprojWarps) {
+    for (int v = warp; v < items; v += kStreamWarps) {
         const int m = v / nb, b = v % nb;
         float4 x4;
         if (keep) {
@@ -270,20 +264,20 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
     if (owner) descale = __uint_as_float(static_cast<unsigned int>(254 - up_exp(em)) << 23);
     }
     __syncthreads();
-    for (int buf = 0; row0 < a.H; buf ^= 1) {
-        const int next = row0 + static_cast<int>(gridDim.x) * kRowsPerGroup;
+    for (int buf = team; row0 < a.H; buf ^= teams == 1) {
+        const int next = row0 + stride;
         const size_t o = static_cast<size_t>(em) * a.H + row0 + er;
         __nv_bfloat16 res = __ushort_as_bfloat16(0);        // requested before the product and kept as read: a conversion here would wait for it
         if (owner && !a.overwrite) res = a.x[o];
         float d[NT][4];
         mw.group(row0, next < a.H ? next : -1, xq, ldx, 3 * a.M, d);
-        // two tile buffers: the barrier of the next group separates this group's readers from the writers after it
+        // one team: two tile buffers, and the barrier of the next group separates this group's readers from the writers after it
         float* tl = tiles + buf * kTiles;
         mw.store(tl, d);
-        __syncthreads();
+        asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory");
         tr.mark(2);
         if (owner) {
-            const float v = Stream::result(tl, kOprojWarps, er, em, descale);
+            const float v = Stream::result(tl, kStreamWarps, er, em, descale);
             if (a.partial_out != nullptr) {
                 a.partial_out[o] = v;
             } else {
@@ -291,6 +285,7 @@ __global__ void __launch_bounds__(256, 2) oproj_allreduce_mma_kernel(OProjArgs a
                 a.x[o] = __float2bfloat16_rn(a.overwrite ? sum : __bfloat162float(res) + sum);
             }
         }
+        if (teams == 2 && next < a.H) asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory");
         row0 = next;
     }
     tr.mark(3);
@@ -376,12 +371,15 @@ static int launch_oproj_mma(const OProjArgs& a, int mode, cudaStream_t st) {
     if (base > all) return -1;
     const size_t kept = base + sizeof(float) * a.M * a.K;
     const int keep = mode != 3 && kept <= (base <= half ? half : all) ? 1 : 0;
+    // what leaves room for two CTAs per SM runs as two; staged terms that do not are shared by the two teams of one CTA (in one
+    // team, two groups follow each other there: an unsharded layer of four rows took 72 us, 59.5 with two)
+    const int teams = mode == 3 && base > half ? 2 : 1, items = (groups + teams - 1) / teams;
     const int resident = sm_count() * (base <= half ? 2 : 1);
-    const int rounds = (groups + resident - 1) / resident;
-    const dim3 g((groups + rounds - 1) / rounds), b(256);                // as few CTAs as the rounds need: each stages the input once
+    const int rounds = (items + resident - 1) / resident;
+    const dim3 g((items + rounds - 1) / rounds), b(256 * teams);         // as few CTAs as the rounds need: each stages the input once
     auto go = [&](auto kernel) { return launch(kernel, g, b, keep ? kept : base, st, a, keep); };
     // windows of one warp per group: the ring holds two, four or (wide K) eight of them, six beside 24 columns
-    const int wpw = (a.K / kWin + kOprojWarps - 1) / kOprojWarps;
+    const int wpw = (a.K / kWin + kStreamWarps - 1) / kStreamWarps;
     if (nt == 1) {
         auto by_mode = [&](auto plain, auto gated, auto merge, auto staged) { return mode == 0 ? go(plain) : (mode == 1 ? go(gated) : (mode == 2 ? go(merge) : go(staged))); };
         if (wpw <= 2) return by_mode(oproj_allreduce_mma_kernel<1, 0, 2>, oproj_allreduce_mma_kernel<1, 1, 2>, oproj_allreduce_mma_kernel<1, 2, 2>, oproj_allreduce_mma_kernel<1, 3, 2>);

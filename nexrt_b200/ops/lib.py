@@ -94,9 +94,8 @@ _PROTOTYPES = {
     "nexrt_moe_dense_act": [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp],
     "nexrt_planes_residual": [vp, vp, vp, c_int64, ci, vp],
     "nexrt_gdn_chunk": [vp] * 14 + [ci] * 9 + [vp],
-    "nexrt_rows_norm_split": [vp, vp, vp, vp, ci, ci, cf, vp],
-    "nexrt_tc_rows_gemm": [vp, vp, vp, vp, vp, ci, ci, ci, ci, vp, vp],
-    "nexrt_gdn_front_tail": [vp] * 12 + [ci] * 7 + [vp],
+    "nexrt_gdn_front_rows": [vp] * 15 + [ci] * 6 + [cf, vp],
+    "nexrt_attn_front_rows": [vp] * 10 + [ci] * 7 + [cf, vp],
     "nexrt_tc_router_logits": [vp] * 6 + [ci] * 5 + [cf, vp, vp, vp],
     "nexrt_moe_router_topk": [vp, ci, ci, vp, vp, vp, ci, ci, ci, vp],
     "nexrt_lmhead_sample_from_logits": [vp] * 6 + [ci] * 6 + [CH, cu, ci, vp],
@@ -164,6 +163,9 @@ def _install_optional(lib) -> None:
 
 class KernelError(RuntimeError):
     pass
+
+
+NOT_SUPPORTED = 801    # cudaErrorNotSupported: the form asked for does not cover this shape, nothing was launched
 
 
 def check(err: int, what: str) -> None:
