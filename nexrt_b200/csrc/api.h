@@ -157,7 +157,11 @@ int nexrt_planes_allreduce_residual(void* x, const void* y, int64_t n, int kspli
 int nexrt_norm_rows(const void* x, const void* gamma, void* xq, void* sx, void* xn, void* planes, int K, int T, float eps, int terms, void* stream);
 int nexrt_gdn_gate_quant(const void* o, const void* z, const void* gnorm_w, void* xq, void* sx, int K, int T, float eps, int terms, void* stream);
 int nexrt_moe_dense_act(const void* gu, const void* ids, const void* wts, void* hq, void* hs, int I, int S, int T, int n_total, int ksplit, int terms, void* stream);   /* gu: [ksplit][T][n_total * 2I] */
-int nexrt_moe_mark_used(const void* ids, void* used, int n_ids, int n_total, void* stream);   /* used[e] = 1 for every routed expert id */
+int nexrt_moe_plan(const void* ids, void* items, void* n_items, void* pair_row, void* out_row, int S, int T, int n_total, int terms, void* stream);
+int nexrt_moe_gather(const void* xq, const void* sx, const void* pair_row, void* xp, void* sp, int pairs, int T, int K, int terms, void* stream);
+int nexrt_moe_group_gemm(const void* w, const void* w_s, const void* xp, const void* sp, void* out, const void* items, const void* n_items, const void* out_row,
+                         int pairs, int n_total, int R, int K, int terms, int* status, void* stream);
+int nexrt_moe_pair_act(const void* gu, const void* out_row, const void* wts, void* hq, void* hs, int I, int S, int T, int terms, void* stream);   /* used[e] = 1 for every routed expert id */
 int nexrt_planes_residual(void* x, const void* y, void* sum_out, int64_t n, int ksplit, void* stream);
 int nexrt_gdn_chunk(const void* pre, const void* xn, const void* ba_w, const void* conv_w, const void* a_log, const void* dt_bias, const void* ctl,
                     void* conv_ring, void* qkv, void* z, void* beta, void* g, void* state_ring, void* out, int H, int R, int C, int nv, int nqk, int T,

@@ -2,8 +2,7 @@
 // projections, router and experts are tcgen05 GEMMs over all rows (tc_gemm.cu), so every weight is streamed once per
 // chunk.  Here: embedding rows from an id list, the control-block table that gives each 8-row attention sub-step its
 // base position, rmsnorm + quantisation of the chunk rows, the GDN layer's conv / gates / delta rule over the whole
-// chunk, the GDN output gate + quantisation, the expert activation of the dense expert product, the skip list of
-// unused experts, and the residual add over K-split planes with or without the tensor-parallel all-reduce.
+// chunk, the GDN output gate + quantisation, the expert activation of a dense expert product, and the residual add over K-split planes with or without the tensor-parallel all-reduce.
 //
 // The reference has no counterpart: its prefill runs inside SGLang (nex_n2_5_pro/sglang_prefill/bridge.py:310-398).
 #include <cuda_fp8.h>
@@ -127,13 +126,6 @@ __global__ void __launch_bounds__(256) moe_dense_act_kernel(const float* __restr
     const float v[4] = {silu_f(gt.x) * up.x * wt, silu_f(gt.y) * up.y * wt, silu_f(gt.z) * up.z * wt, silu_f(gt.w) * up.w * wt};
     quant_block4<P>(v, hq + (static_cast<size_t>(m) * n_total + e) * I + b * 128, hs + (static_cast<size_t>(m) * n_total + e) * nb + b, lane,
                     static_cast<size_t>(T) * n_total * I, static_cast<size_t>(T) * n_total * nb);
-}
-
-__global__ void moe_mark_used_kernel(const int* __restrict__ ids, int* __restrict__ used, int n_ids, int n_total) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_ids) used[min(max(ids[i], 0), n_total - 1)] = 1;
 }
 
 // out = sum of the K-split planes y[ks][n]; with x != null the sum is added to the bf16 residual rows instead
@@ -551,14 +543,6 @@ int nexrt_moe_dense_act(const void* gu, const void* ids, const void* wts, void* 
     return terms == 1 ? go(moe_dense_act_kernel<1>) : terms == 2 ? go(moe_dense_act_kernel<2>) : go(moe_dense_act_kernel<3>);
 }
 
-
-int nexrt_moe_mark_used(const void* ids, void* used, int n_ids, int n_total, void* stream) {
-    if (n_ids < 1 || n_total < 1) return cudaErrorInvalidValue;
-    auto s = static_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaMemsetAsync(used, 0, sizeof(int) * n_total, s);
-    if (e != cudaSuccess) return e;
-    return launch(moe_mark_used_kernel, dim3((n_ids + 255) / 256), dim3(256), 0, s, static_cast<const int*>(ids), static_cast<int*>(used), n_ids, n_total);
-}
 
 int nexrt_planes_residual(void* x, const void* y, void* sum_out, int64_t n, int ksplit, void* stream) {
     if (n < 4 || n % 4 || ksplit < 1) return cudaErrorInvalidValue;

@@ -81,7 +81,10 @@ _PROTOTYPES = {
     "nexrt_act_quant": [vp, ci, ci, vp, cf, vp, vp, ci, ci, ci, vp],
     "nexrt_tc_gemm_bf16_ex": [vp, c_int64, vp, c_int64, vp, ci, ci, ci, ci, ci, vp, vp],
     "nexrt_tc_gemm_fp8_ex": [vp, vp, c_int64, vp, vp, vp, ci, ci, ci, ci, ci, ci, ci, vp, ci, vp, vp],
-    "nexrt_moe_mark_used": [vp, vp, ci, ci, vp],
+    "nexrt_moe_plan": [vp] * 5 + [ci] * 4 + [vp],
+    "nexrt_moe_gather": [vp] * 5 + [ci] * 4 + [vp],
+    "nexrt_moe_group_gemm": [vp] * 8 + [ci] * 5 + [vp, vp],
+    "nexrt_moe_pair_act": [vp] * 5 + [ci] * 4 + [vp],
     "nexrt_prefill_embed": [vp, vp, vp, vp, ci, ci, ci, vp],
     "nexrt_prefill_ctl": [vp, vp, ci, ci, vp],
     "nexrt_prefill_advance": [vp, ci, vp, cu, vp],

@@ -7,10 +7,9 @@ tokens.  Here a chunk of ``T`` rows goes through each layer in one pass:
 * every projection (GDN / attention fronts, out-projections, router, expert gate/up and down) is one tcgen05 GEMM
   over all ``T`` rows (``csrc/tc_gemm.cu``): e4m3 activations with one scale per row and 128 columns, the
   checkpoint's block-scaled FP8 weights, fp32 accumulation - every weight byte is read once per chunk;
-* the experts run **dense**: the gate/up GEMM multiplies the chunk by all ``E + 1`` experts (with 64 rows x 10
-  routes nearly every expert is used anyway, and the FP8 tensor cores make the extra columns cheaper than a
-  gather), a small kernel turns the routed ``(row, expert)`` pairs into quantised ``h`` and leaves a zero scale
-  everywhere else, and the down GEMM walks ``K = (E + 1) * I`` split over CTAs;
+* the experts run **grouped** (``csrc/tc_group.cu``): the chunk's ``(row, expert)`` pairs are sorted by expert, a
+  persistent tcgen05 GEMM multiplies every used expert by its own rows, and the down products land in one plane per
+  slot that the residual add sums;
 * the GDN layer's conv ring, gates and delta rule run over the whole chunk in two kernels (``csrc/prefill.cu``: the
   step kernels' arithmetic, the recurrent state kept in registers along the chunk);
 * causal attention reuses the multi-row decode kernel eight rows at a time: the chunk's q / gate / k rows are scattered
@@ -117,15 +116,15 @@ class WidePrefill:
         self.logits = z(2 * self.router_ksplit, T, self.rows_pad)
         self.moe_logits, self.moe_ids, self.moe_wts = z(T, cfg.n_experts + 1), z(T, self.S, dtype=i32), z(T, self.S)
         I = spec.inter
-        self.used = z(self.n_total, dtype=i32)
-        # K split of the gate/up product: 1 (two half-length CTAs per tile fill the last wave better but write and re-read a
-        # second 34 MB plane: measured 4 % slower per chunk at 64 rows)
-        self.up_ksplit = 1
-        self.gu = z(self.up_ksplit, P * T, self.n_total * 2 * I)
-        self.hq, self.hs = torch.zeros(P * T, self.n_total * I, dtype=FP8, device=dev), z(P * T, self.n_total * I // 128)
-        # K split of the expert down product: at most 64 K blocks per CTA, and about two CTAs per SM over the grid
-        self.down_ksplit = down_split(self.n_total * I // 128, (H // 128) * ((P * T + 63) // 64), c.n_cta)
-        self.y = z(max(self.down_ksplit, 1), P * T, H)
+        # experts: the chunk's (row, slot) pairs sorted by expert, their rows, gate | up and activations (csrc/tc_group.cu)
+        self.pairs = T * self.S
+        self.items, self.n_items = z(self.pairs, 4, dtype=i32), z(1, dtype=i32)
+        self.pair_row, self.out_row = z(self.pairs, dtype=i32), z(self.pairs, dtype=i32)
+        self.xp, self.sp = torch.zeros(P * self.pairs, H, dtype=FP8, device=dev), z(self.pairs, H // 128)
+        self.gu = z(self.pairs, 2 * I)
+        self.hq, self.hs = torch.zeros(P * self.pairs, I, dtype=FP8, device=dev), z(self.pairs, I // 128)
+        # what is added to the residual rows: one plane [T][H] per activation term (out-projections) or per slot (experts)
+        self.y = z(max(P, self.S) * T, H)
         # tensor parallel: the chunk's partial sums are all-reduced inside the residual kernel over a symmetric inbox of its
         # own (8 bytes per value of the chunk and half: data vectors, then one flag word per CTA); it shares the engine's
         # sequence word and status, so its tags never collide with the decode steps' and a failure stops both
@@ -143,15 +142,14 @@ class WidePrefill:
         self.graph = None
 
     # ---- one chunk ---------------------------------------------------------------------------------------------
-    def _finish(self, ksplit: int) -> None:
-        """x += (all-reduced) sum of the projection's K-split planes, each of which holds one row block per activation term."""
+    def _finish(self, planes: int) -> None:
+        """x += (all-reduced) sum of the first ``planes`` planes ``[T][H]`` of ``y``."""
         c, lib, st = self.eng.ctx, self.eng.ctx.lib, self.eng.ctx.stream()
         n = self.T * self.eng.cfg.hidden
-        ksplit *= self.P
         if self.channel is None:
-            check(lib.nexrt_planes_residual(ptr(self.x), ptr(self.y), None, n, ksplit, st), "planes_residual")
+            check(lib.nexrt_planes_residual(ptr(self.x), ptr(self.y), None, n, planes, st), "planes_residual")
             return
-        check(lib.nexrt_planes_allreduce_residual(ptr(self.x), ptr(self.y), n, ksplit, self.channel.ref, self.site, st), "planes_allreduce_residual")
+        check(lib.nexrt_planes_allreduce_residual(ptr(self.x), ptr(self.y), n, planes, self.channel.ref, self.site, st), "planes_allreduce_residual")
         self.site += 1
 
     def _gdn(self, m) -> None:
@@ -173,8 +171,8 @@ class WidePrefill:
         )
         oq, os_ = self.oq[: P * T * K].view(P * T, K), self.os[: P * T * (K // 128)].view(P * T, K // 128)
         check(lib.nexrt_gdn_gate_quant(ptr(self.gdn_out), ptr(self.gdn_z), ptr(w["gnorm_w"]), ptr(oq), ptr(os_), K, T, cfg.rms_eps, P, st), "gdn_gate_quant")
-        fp8_gemm(w["out_w"], w["out_s"], oq, os_, out=self.y[0], status=c.status)
-        self._finish(1)
+        fp8_gemm(w["out_w"], w["out_s"], oq, os_, out=self.y[: P * T], status=c.status)
+        self._finish(P)
 
     def _attn(self, m: FullAttn) -> None:
         eng, T = self.eng, self.T
@@ -214,8 +212,8 @@ class WidePrefill:
             cur.wait_stream(self.side[j])
         oq, os_ = self.oq[: P * T * K].view(P * T, K), self.os[: P * T * (K // 128)].view(P * T, K // 128)
         check(lib.nexrt_act_quant(ptr(self.attn_out), 1, K, None, cfg.rms_eps, ptr(oq), ptr(os_), T, K, P, st), "act_quant")
-        fp8_gemm(w["out_w"], w["out_s"], oq, os_, out=self.y[0], status=c.status)
-        self._finish(1)
+        fp8_gemm(w["out_w"], w["out_s"], oq, os_, out=self.y[: P * T], status=c.status)
+        self._finish(P)
 
     def _moe(self, moe) -> None:
         eng, T = self.eng, self.T
@@ -230,17 +228,16 @@ class WidePrefill:
         bf16_gemm_split(w["router_w_pad"], self.planes[:, H:], self.logits[ks:], ks, status=c.status)
         check(lib.nexrt_moe_router_topk(ptr(self.logits), 2 * ks, self.rows_pad, ptr(self.moe_logits), ptr(self.moe_ids), ptr(self.moe_wts),
                                         cfg.n_experts, cfg.top_k, T, st), "moe_router_topk")
-        # experts, dense: gate/up of every expert for every row, activation of the routed pairs, down over all experts
-        # (experts no row of the chunk routes to are skipped: their weights are not read)
-        check(lib.nexrt_moe_mark_used(ptr(self.moe_ids), ptr(self.used), T * S, n_total, st), "moe_mark_used")
-        fp8_gemm_split(w["w13"].view(n_total * 2 * I, H), w["w13_s"].view(-1, H // 128), self.xq, self.sx, self.gu, ksplit=self.up_ksplit, used=self.used, used_rows=2 * I,
-                       status=c.status)
-        self.hq.view(torch.uint8).zero_()
-        self.hs.zero_()
-        check(lib.nexrt_moe_dense_act(ptr(self.gu), ptr(self.moe_ids), ptr(self.moe_wts), ptr(self.hq), ptr(self.hs), I, S, T, n_total, self.up_ksplit * P, P, st),
-              "moe_dense_act")
-        fp8_gemm_split(w["w2"].view(n_total * H, I), w["w2_s"], self.hq, self.hs, self.y, ksplit=self.down_ksplit, group_k=I, group_rows=H, used=self.used, status=c.status)
-        self._finish(self.down_ksplit)
+        # experts: every expert's weights against the rows routed to it; the down product writes one plane of y per slot
+        pairs = self.pairs
+        check(lib.nexrt_moe_plan(ptr(self.moe_ids), ptr(self.items), ptr(self.n_items), ptr(self.pair_row), ptr(self.out_row), S, T, n_total, P, st), "moe_plan")
+        check(lib.nexrt_moe_gather(ptr(self.xq), ptr(self.sx), ptr(self.pair_row), ptr(self.xp), ptr(self.sp), pairs, T, H, P, st), "moe_gather")
+        check(lib.nexrt_moe_group_gemm(ptr(w["w13"]), ptr(w["w13_s"]), ptr(self.xp), ptr(self.sp), ptr(self.gu), ptr(self.items), ptr(self.n_items), None,
+                                       pairs, n_total, 2 * I, H, P, ptr(c.status), st), "moe_group_gemm")
+        check(lib.nexrt_moe_pair_act(ptr(self.gu), ptr(self.out_row), ptr(self.moe_wts), ptr(self.hq), ptr(self.hs), I, S, T, P, st), "moe_pair_act")
+        check(lib.nexrt_moe_group_gemm(ptr(w["w2"]), ptr(w["w2_s"]), ptr(self.hq), ptr(self.hs), ptr(self.y), ptr(self.items), ptr(self.n_items), ptr(self.out_row),
+                                       pairs, n_total, H, I, P, ptr(c.status), st), "moe_group_gemm")
+        self._finish(S)
 
     def _chunk(self) -> None:
         """All layers over the rows named by ``self.ids`` at the engine's committed length, which then advances by T."""

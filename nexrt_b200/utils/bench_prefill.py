@@ -57,9 +57,10 @@ def stage_costs(eng, T: int, replays: int = 10) -> dict:
         "residual": lambda n, a: n == "nexrt_planes_residual",
         "router_gemms": lambda n, a: n == "nexrt_tc_gemm_bf16_ex",
         "router_topk": lambda n, a: n == "nexrt_moe_router_topk",
-        "expert_up_gemm": lambda n, a: n == "nexrt_tc_gemm_fp8_ex" and a[12] == 0 and a[13] is not None,
-        "dense_act": lambda n, a: n == "nexrt_moe_dense_act",
-        "expert_down_gemm": lambda n, a: n == "nexrt_tc_gemm_fp8_ex" and a[12] != 0,
+        "plan_gather": lambda n, a: n in ("nexrt_moe_plan", "nexrt_moe_gather"),
+        "expert_up_gemm": lambda n, a: n == "nexrt_moe_group_gemm" and a[7] is None,
+        "pair_act": lambda n, a: n == "nexrt_moe_pair_act",
+        "expert_down_gemm": lambda n, a: n == "nexrt_moe_group_gemm" and a[7] is not None,
     }
     prompt = synthetic_prompt(cfg.vocab, 2 * T, seed=1)
     out = {}

@@ -1,0 +1,63 @@
+"""Grouped experts of a prefill chunk: the plan against a host sort, the persistent GEMM against float64, with experts nobody is
+routed to, experts of more pairs than one item holds, CTAs with no, one and many tiles, and one and several K blocks."""
+
+import pytest
+import torch
+
+from nexrt_b200.ops.lib import check, load, ptr
+from nexrt_b200.quant import dequantize_blockwise, quantize_blockwise
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _ids(g, T, S, E, skew):
+    """Distinct routed experts per row, the shared expert (id E) last; ``skew``: every row picks the same ones."""
+    rows = [torch.randperm(E, generator=g)[: S - 1].sort().values if not (skew and t) else None for t in range(T)]
+    return torch.stack([torch.cat([r if r is not None else rows[0], torch.tensor([E])]) for r in rows]).to(torch.int32)
+
+
+@pytest.mark.parametrize("T,S,E,R,K,terms,skew", [(16, 2, 1, 128, 128, 1, False), (16, 5, 16, 512, 1024, 3, False), (24, 11, 512, 256, 512, 3, False),
+                                                  (64, 11, 40, 256, 384, 2, False), (128, 11, 512, 4096, 128, 3, False), (128, 4, 12, 256, 256, 1, True),
+                                                  (128, 11, 30, 1024, 256, 3, True)])
+def test_plan_and_group_gemm(T, S, E, R, K, terms, skew):
+    g = torch.Generator().manual_seed(T + S + E)
+    ids = _ids(g, T, S, E, skew)
+    lib, st, pairs, n_total, NP = load(), torch.cuda.current_stream().cuda_stream, T * S, E + 1, 32 // terms
+    i32 = lambda *s: torch.full(s, -1, dtype=torch.int32, device=DEV)
+    items, n_items, pair_row, out_row = i32(pairs, 4), i32(1), i32(pairs), i32(pairs)
+    check(lib.nexrt_moe_plan(ptr(ids.to(DEV)), ptr(items), ptr(n_items), ptr(pair_row), ptr(out_row), S, T, n_total, terms, st), "plan")
+    want = sorted((int(ids[m, s]), m, s) for m in range(T) for s in range(S))
+    assert pair_row.tolist() == [m for _, m, _ in want]
+    assert out_row.tolist() == [s * T + m for _, m, s in want]
+    tiles, first = [], 0
+    for e in range(n_total):
+        n = sum(1 for w in want if w[0] == e)
+        tiles += [[e, first + i, min(NP, n - i), 0] for i in range(0, n, NP)]
+        first += n
+    assert int(n_items.item()) == len(tiles) and items[: len(tiles)].tolist() == tiles
+
+    gd = torch.Generator(device=DEV).manual_seed(K + R)
+    wq, ws = quantize_blockwise(torch.randn(n_total, R, K, device=DEV, generator=gd) * 0.03)
+    xq = (torch.randn(terms * T, K, device=DEV, generator=gd) * 100).to(torch.float8_e4m3fn)
+    sx = torch.rand(terms * T, K // 128, device=DEV, generator=gd) * 0.02 + 0.001
+    xp, sp = torch.zeros(terms * pairs, K, dtype=torch.uint8, device=DEV), torch.zeros(pairs, K // 128, device=DEV)
+    check(lib.nexrt_moe_gather(ptr(xq), ptr(sx), ptr(pair_row), ptr(xp), ptr(sp), pairs, T, K, terms, st), "gather")
+    rows = pair_row.long()
+    assert torch.equal(sp, sx[rows])
+    assert torch.equal(xp.view(pairs, terms, K), torch.stack([xq.view(torch.uint8)[p * T + rows] for p in range(terms)], 1))
+    x = sum(xq.double().view(terms, T, K)[p][rows] * 16.0**-p for p in range(terms)) * sp.double().repeat_interleave(128, 1)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for mapped in (False, True):
+        out = torch.full((pairs, R), float("nan"), device=DEV)
+        check(lib.nexrt_moe_group_gemm(ptr(wq), ptr(ws), ptr(xp), ptr(sp), ptr(out), ptr(items), ptr(n_items), ptr(out_row) if mapped else None, pairs, n_total, R, K,
+                                       terms, ptr(status), st), "group_gemm")
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        got = out[out_row.long()] if mapped else out
+        for e in range(n_total):
+            sel = [i for i, w in enumerate(want) if w[0] == e]
+            if sel:
+                w = dequantize_blockwise(wq[e], ws[e]).double()
+                y, mag = x[sel] @ w.T, x[sel].abs() @ w.abs().T
+                assert ((got[sel].double() - y).abs() <= 1e-5 * mag).all(), (e, ((got[sel].double() - y).abs() / mag).max())   # fp32 sums of up to K exact products
