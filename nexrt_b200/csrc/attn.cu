@@ -22,9 +22,12 @@
 #include "gemv_cta.cuh"
 #include "mma_gemv.cuh"
 #include "attn_mma.cuh"
+#include "attn_stream.cuh"
 #include "ll.cuh"
 
 #include <cooperative_groups.h>
+
+#include <climits>
 
 namespace nexrt {
 
@@ -614,11 +617,13 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(AttnDecodeArgs a) {
 // Replaces wgmma_fd4_mega's software grid barrier + combine (nex_n2_5_pro/kernels/full_attn/
 // nex_n2_5_pro_attn_fd4_wgmma_ctypes.cu:98-118,389-401) with hardware cluster barriers; nothing here spins.
 namespace cg = cooperative_groups;
+// Keys from which the streaming form works instead of the cluster kernel (see stream_min_keys).
+constexpr int kStreamFrom = 2048, kStreamFromTwoHeads = 5120;
 constexpr int kClusterCtas = 8;       // portable cluster size
 constexpr int kClusterCtasWide = 16;  // the largest (non-portable) size: twice the warps, so one 16-key tile per warp up to 2048 keys
 
 template <int HD, int CL>
-__global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs a) {
+__global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs a, int max_keys) {
     constexpr int RP = kRowsPerPassMma, NW = 8, EL = HD / 32, SL = HD / CL;
     constexpr int kKeysPerCluster = CL * 8 * 16;   // one 16-key tile per warp
     extern __shared__ __align__(16) float smem[];
@@ -663,7 +668,7 @@ __global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs
     if (early) {
         C0 = *reinterpret_cast<const volatile int*>(a.ctl + kCtlCommittedLen);
         ranges();
-        if (cidx < n_act) {
+        if (cidx < n_act && win_hi - win_lo <= max_keys) {
             // rows of this warp's first tile that earlier steps wrote: one lane per 128-byte line
             constexpr int LINES = HD * 2 / 128;
             const int t0 = lo + 16 * warp, t1 = min(min(t0 + 16, hi), C0);
@@ -682,7 +687,7 @@ __global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs
         C0 = a.ctl[kCtlCommittedLen];
         ranges();
     }
-    if (cidx >= n_act) { tr.mark(3); return; }          // whole clusters leave: no barrier is left half attended
+    if (cidx >= n_act || win_hi - win_lo > max_keys) { tr.mark(3); return; }   // whole clusters leave: no barrier is left half attended
 
     const int r0 = static_cast<int>(blockIdx.z) * RP, nr = min(RP, rows - r0);
     // one cluster and no context parallelism: the cluster's combine is the final result; otherwise the clusters' partials
@@ -926,6 +931,401 @@ __global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs
     tr.mark(3);
 }
 
+// ---- streaming form (attn_stream.cuh) and its merge ----------------------------------------------------------------------
+// Both are launched behind the cluster kernel where the cache can hold more than `min_keys` keys, and the committed length
+// decides on the device which of them works: the cluster kernel up to min_keys, these two above (a launch that leaves at once
+// costs the step 0.6 us).  All of them wait for their predecessor before they leave, so the chain of dependent launches holds
+// whichever works.
+//
+// One B200, one rank's heads (4 over one kv head): one row at 200K keys 60.9 us in the cluster kernel -> 41 + 4 us (205 MB,
+// 5.0 TB/s); eight rows at 32K keys, four passes over K and V, 61.7 -> 23.5 + 4.1 us.  Code that runs once is kept rolled where
+// that needs no indexed registers: the unrolled prologue and score loop cost 6 us of instruction fetches a launch.
+template <int NTR, int WR>
+__global__ void __launch_bounds__(stream_rings<WR>() * WR * 32, 1) attn_stream_kernel(AttnDecodeArgs a, int min_keys) {
+    constexpr int HD = kStreamHd, NR = stream_rings<WR>(), NW = NR * WR, RW = 8 * NTR, D = kTileDepth, KS = HD / 16;
+    extern __shared__ __align__(16) uint8_t stream_smem[];
+    TraceCta tr;
+    tr.begin(kTrAttnDecode);
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ring = warp / WR, wr = warp % WR, g = lane >> 2, t = lane & 3;
+    const int kv = blockIdx.y, G = a.nq / a.kvh, rows_all = a.M * G, r0 = static_cast<int>(blockIdx.z) * RW * WR, rows = min(RW * WR, rows_all - r0);
+    const bool early = (a.flags & 8) != 0;
+    uint8_t* stages = stream_smem + ring * D * kTileStage;
+    uint32_t* qf = reinterpret_cast<uint32_t*>(stream_smem + NR * D * kTileStage);                // [WR][KS][32 lanes][4 NTR]
+    uint4* k_s = reinterpret_cast<uint4*>(qf + WR * KS * 32 * 4 * NTR);                           // [M][HD] bf16: K rows of this step
+    float* scratch = reinterpret_cast<float*>(k_s + a.M * 32) + warp * HD;                        // this warp's row; at the end the rings' weights
+    float2* rope_s = reinterpret_cast<float2*>(reinterpret_cast<float*>(k_s + a.M * 32) + NW * HD);   // [M][rotary / 2] cos, sin of the rows' positions
+    const int half = a.rotary / 2;
+    const __nv_bfloat16* kc = a.k_cache + static_cast<size_t>(kv) * a.cache_len * HD;
+    const __nv_bfloat16* vc = a.v_cache + static_cast<size_t>(kv) * a.cache_len * HD;
+
+    int C0 = 0, n_keys = 0, n_act = 1, lo = 0, hi = 0, n_tiles = 0;
+    auto ranges = [&]() {
+        n_keys = min(C0 + a.M, a.cache_len);
+        n_act = max(1, min(static_cast<int>(gridDim.x), (n_keys + NR * kTileKeys - 1) / (NR * kTileKeys)));
+        const int tiles = (n_keys + kTileKeys - 1) / kTileKeys, per = (tiles + n_act - 1) / n_act * kTileKeys;      // whole tiles per CTA
+        lo = min(n_keys, static_cast<int>(blockIdx.x) * per);
+        hi = min(n_keys, lo + per);
+        n_tiles = max(0, (hi - lo + kTileKeys - 1) / kTileKeys - ring + NR - 1) / NR;             // tiles ring, ring + NR, ... of the CTA
+    };
+    // requests tile i of the ring: the warps of the ring share its rows
+    auto request = [&](int i) {
+        if (i < n_tiles) {
+            const int t0 = lo + kTileKeys * (ring + NR * i);
+            uint8_t* st = stages + (i % D) * kTileStage;
+#pragma unroll
+            for (int r = wr; r < kTileKeys; r += WR) {
+                const int p = t0 + r;
+                const size_t off = static_cast<size_t>(min(p, n_keys - 1)) * HD + lane * 8;
+                cp_async16_zfill(st + r * kTileRow + lane * 16, kc + off, p < C0 && p < hi);
+                cp_async16_zfill(st + kTileHalf + r * kTileRow + lane * 16, vc + off, p < hi);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto rotations = [&]() {
+        for (int i = threadIdx.x; i < a.M * half; i += blockDim.x) {
+            const int m = i / half, f = i % half;
+            float2 r;
+            if (a.rope_table != nullptr && C0 + m < a.cache_len) r = a.rope_table[static_cast<size_t>(C0 + m) * half + f];
+            else sincosf(static_cast<float>(C0 + m) * a.inv_freq[f], &r.y, &r.x);
+            rope_s[i] = r;
+        }
+    };
+    int asked = 0;
+    if (early) {
+        C0 = *reinterpret_cast<const volatile int*>(a.ctl + kCtlCommittedLen);
+        ranges();
+        // tiles of earlier steps' rows only: the rows of this step are being written
+        if (n_keys > min_keys)
+            while (asked < D && asked < n_tiles && lo + kTileKeys * (ring + NR * asked + 1) <= C0) request(asked++);
+        rotations();
+    }
+    const float4 qg0 = *reinterpret_cast<const float4*>(a.qn + lane * 8), qg1 = *reinterpret_cast<const float4*>(a.qn + lane * 8 + 4);
+    const float4 kg0 = *reinterpret_cast<const float4*>(a.kn + lane * 8), kg1 = *reinterpret_cast<const float4*>(a.kn + lane * 8 + 4);
+    for (int i = threadIdx.x; i < WR * KS * 32 * 4 * NTR; i += blockDim.x) qf[i] = 0u;            // rows that do not exist
+    pdl_wait();
+    tr.mark(1);
+    if (!early) {
+        C0 = a.ctl[kCtlCommittedLen];
+        ranges();
+    }
+    if (n_keys <= min_keys || lo >= hi) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        tr.mark(3);
+        return;
+    }
+    while (asked < D) request(asked++);
+    if (!early) rotations();
+    // ---- q and new-k normalisation + RoPE, one warp per vector (the arithmetic of attn_decode_kernel)
+    const float qscale = rsqrtf(static_cast<float>(HD)) * 1.4426950408889634f;
+    // A lane holds the eight dims from 8 lane on: two of its row's fragment pieces (see attn_mma_stage_q).  The values of a
+    // warp's next vector are requested before the current one is worked on; kept rolled, the code of all of it is fetched once.
+    const int n_vec = rows + a.M;
+    auto fetch = [&](int v, float4& x, float4& y) {
+        if (v >= n_vec) return;
+        const int row = r0 + v;
+        const float* src = v < rows ? a.q_raw + (static_cast<size_t>(row / G) * a.nq + kv * G + row % G) * HD : a.k_raw + (static_cast<size_t>(v - rows) * a.kvh + kv) * HD;
+        x = *reinterpret_cast<const float4*>(src + lane * 8);
+        y = *reinterpret_cast<const float4*>(src + lane * 8 + 4);
+    };
+    float4 nx = make_float4(0.f, 0.f, 0.f, 0.f), ny = nx;
+    fetch(warp, nx, ny);
+    __syncthreads();
+#pragma unroll 1
+    for (int v = warp; v < n_vec; v += NW) {
+        const bool is_q = v < rows;
+        const int m = is_q ? (r0 + v) / G : v - rows;
+        float e[8] = {nx.x, nx.y, nx.z, nx.w, ny.x, ny.y, ny.z, ny.w};
+        fetch(v + NW, nx, ny);
+        const float4 g0 = is_q ? qg0 : kg0, g1 = is_q ? qg1 : kg1;
+        const float gm[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss = fmaf(e[i], e[i], ss);
+        const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(HD) + a.eps);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            e[i] = e[i] * inv * gm[i];
+            scratch[lane * 8 + i] = e[i];
+        }
+        __syncwarp();
+        if (lane * 8 < a.rotary) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int d = lane * 8 + i;
+                if (d < a.rotary) {
+                    const float2 cs = rope_s[m * half + (d < half ? d : d - half)];
+                    e[i] = e[i] * cs.x + (d < half ? -scratch[d + half] : scratch[d - half]) * cs.y;
+                }
+            }
+        }
+        __syncwarp();
+        if (is_q) {
+            const int vr = v % RW, ln = (vr & 7) * 4 + ((lane * 8 & 63) >> 4), ks0 = (lane >> 3) * 4 + (lane & 1) * 2;
+            uint4* f = reinterpret_cast<uint4*>(qf + static_cast<size_t>(v / RW) * KS * 32 * 4 * NTR);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint4 w;                                              // hi (dims 0, 1), hi (2, 3), lo, lo of this K step
+                split_pair(e[4 * h] * qscale, e[4 * h + 1] * qscale, w.x, w.z);
+                split_pair(e[4 * h + 2] * qscale, e[4 * h + 3] * qscale, w.y, w.w);
+                f[((ks0 + h) * 32 + ln) * NTR + (vr >> 3)] = w;
+            }
+        } else {
+            uint4 w;
+            w.x = pack_bf16(e[0], e[1]); w.y = pack_bf16(e[2], e[3]); w.z = pack_bf16(e[4], e[5]); w.w = pack_bf16(e[6], e[7]);
+            k_s[static_cast<size_t>(m) * 32 + lane] = w;
+            if (blockIdx.x == 0 && blockIdx.z == 0 && C0 + m < a.cache_len)
+                *reinterpret_cast<uint4*>(a.k_cache + (static_cast<size_t>(kv) * a.cache_len + C0 + m) * HD + lane * 8) = w;
+        }
+    }
+    __syncthreads();
+    tr.mark(4);
+
+    // ---- the ring's tiles
+    const uint4* qv = reinterpret_cast<const uint4*>(qf + static_cast<size_t>(wr) * KS * 32 * 4 * NTR);
+    int limit[NTR];
+#pragma unroll
+    for (int n = 0; n < NTR; ++n) {
+        const int rr = wr * RW + n * 8 + g;
+        limit[n] = rr < rows ? C0 + (r0 + rr) / G : -1;                                           // last position the row may see
+    }
+    float o[NTR][KS][4], mx[NTR], l[NTR];
+#pragma unroll
+    for (int n = 0; n < NTR; ++n) {
+        mx[n] = -INFINITY;
+        l[n] = 0.f;
+#pragma unroll
+        for (int j = 0; j < KS; ++j) o[n][j][0] = o[n][j][1] = o[n][j][2] = o[n][j][3] = 0.f;
+    }
+    auto ring_sync = [&]() {
+        if (WR == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + ring), "n"(WR * 32) : "memory");
+    };
+    for (int i = 0; i < n_tiles; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+        ring_sync();
+        const int tile = lo + kTileKeys * (ring + NR * i);
+        const uint8_t* kt = stages + (i % D) * kTileStage;
+        const uint8_t* vt = kt + kTileHalf;
+        // scores of 16 keys: tile + g (column group 0) and tile + 8 + g (group 1) on the N side; hi and lo products apart
+        float sh[2][4], sl[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) sh[h][0] = sh[h][1] = sh[h][2] = sh[h][3] = sl[h][0] = sl[h][1] = sl[h][2] = sl[h][3] = 0.f;
+        const bool fresh = tile + kTileKeys > C0;                                                 // some keys are rows of this step
+#pragma unroll 1
+        for (int b = 0; b < HD / 64; ++b) {
+            uint32_t kr[2][8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4* src = reinterpret_cast<const uint4*>(kt + (h * 8 + g) * kTileRow + b * 128 + t * 32);
+                const uint4 x = src[0], y = src[1];
+                kr[h][0] = x.x; kr[h][1] = x.y; kr[h][2] = x.z; kr[h][3] = x.w; kr[h][4] = y.x; kr[h][5] = y.y; kr[h][6] = y.z; kr[h][7] = y.w;
+                const int p = tile + h * 8 + g;
+                if (fresh && p >= C0 && p < hi) {
+                    const uint4 x2 = k_s[(p - C0) * 32 + b * 8 + t * 2], y2 = k_s[(p - C0) * 32 + b * 8 + t * 2 + 1];
+                    kr[h][0] = x2.x; kr[h][1] = x2.y; kr[h][2] = x2.z; kr[h][3] = x2.w; kr[h][4] = y2.x; kr[h][5] = y2.y; kr[h][6] = y2.z; kr[h][7] = y2.w;
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const uint4 q0 = qv[((b * 4 + s) * 32 + lane) * NTR];
+                uint4 q1 = make_uint4(0u, 0u, 0u, 0u);
+                if (NTR == 2) q1 = qv[((b * 4 + s) * 32 + lane) * NTR + 1];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    mma_bf16_16x8x16(sh[h], q0.x, q1.x, q0.y, q1.y, kr[h][2 * s], kr[h][2 * s + 1]);
+                    mma_bf16_16x8x16(sl[h], q0.z, q1.z, q0.w, q1.w, kr[h][2 * s], kr[h][2 * s + 1]);
+                }
+            }
+        }
+        const int kp[4] = {tile + 2 * t, tile + 2 * t + 1, tile + 8 + 2 * t, tile + 9 + 2 * t};
+        uint32_t ph[NTR][2], pl[NTR][2];
+#pragma unroll
+        for (int n = 0; n < NTR; ++n) {
+            float sv[4] = {sh[0][2 * n] + sl[0][2 * n], sh[0][2 * n + 1] + sl[0][2 * n + 1], sh[1][2 * n] + sl[1][2 * n], sh[1][2 * n + 1] + sl[1][2 * n + 1]};
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (kp[q] > limit[n] || kp[q] >= hi) sv[q] = -INFINITY;
+            float tm = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
+            tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
+            const float mn = fmaxf(mx[n], tm), mu = mn == -INFINITY ? 0.f : mn;
+            const float corr = mx[n] == mn ? 1.f : exp2f(mx[n] - mu);
+            float p[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] = exp2f(sv[q] - mu);
+            l[n] = fmaf(l[n], corr, (p[0] + p[1]) + (p[2] + p[3]));
+            mx[n] = mn;
+            split_pair(p[0], p[1], ph[n][0], pl[n][0]);
+            split_pair(p[2], p[3], ph[n][1], pl[n][1]);
+            // the accumulators of this lane belong to rows 2t and 2t + 1, whose state lives in lanes 8t and 8t + 4
+            const float c0 = __shfl_sync(0xffffffffu, corr, 8 * t), c1 = __shfl_sync(0xffffffffu, corr, 8 * t + 4);
+            if (__any_sync(0xffffffffu, corr != 1.f)) {
+#pragma unroll
+                for (int j = 0; j < KS; ++j) { o[n][j][0] *= c0; o[n][j][1] *= c1; o[n][j][2] *= c0; o[n][j][3] *= c1; }
+            }
+        }
+#pragma unroll
+        for (int blk = 0; blk < HD / 128; ++blk) {
+            uint4 v[4][2];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4* src = reinterpret_cast<const uint4*>(vt + ((q >> 1) * 8 + 2 * t + (q & 1)) * kTileRow + blk * 256 + g * 16);
+                v[q][0] = src[0];
+                v[q][1] = src[8];
+            }
+            // hi products of a few output tiles, then their lo products: back to back, a lo product would wait for the hi
+            // product of the same tile (the instructions are issued in the order written)
+            constexpr int JB = 4 / NTR;
+#pragma unroll
+            for (int j0 = 0; j0 < 8; j0 += JB) {
+                uint32_t av[JB][4];
+#pragma unroll
+                for (int u = 0; u < JB; ++u) {
+                    const int j = j0 + u;
+                    const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+                    auto word = [&](const uint4& q4) { return (j >> 1) == 0 ? q4.x : ((j >> 1) == 1 ? q4.y : ((j >> 1) == 2 ? q4.z : q4.w)); };
+                    av[u][0] = prmt(word(v[0][0]), word(v[1][0]), sel); av[u][1] = prmt(word(v[0][1]), word(v[1][1]), sel);
+                    av[u][2] = prmt(word(v[2][0]), word(v[3][0]), sel); av[u][3] = prmt(word(v[2][1]), word(v[3][1]), sel);
+                }
+#pragma unroll
+                for (int u = 0; u < JB; ++u)
+#pragma unroll
+                    for (int n = 0; n < NTR; ++n) mma_bf16_16x8x16(o[n][blk * 8 + j0 + u], av[u][0], av[u][1], av[u][2], av[u][3], ph[n][0], ph[n][1]);
+#pragma unroll
+                for (int u = 0; u < JB; ++u)
+#pragma unroll
+                    for (int n = 0; n < NTR; ++n) mma_bf16_16x8x16(o[n][blk * 8 + j0 + u], av[u][0], av[u][1], av[u][2], av[u][3], pl[n][0], pl[n][1]);
+            }
+        }
+        ring_sync();                                             // every warp of the ring has read the stage
+        request(i + D);
+    }
+    // ---- this warp's partial into its ring (drained: the last requests were empty), then the rings into the workspace
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    ring_sync();
+    tr.mark(5);
+    float* part = reinterpret_cast<float*>(stages + wr * kTileStage);                             // [RW][HD + 2]
+#pragma unroll
+    for (int n = 0; n < NTR; ++n) {
+        l[n] += __shfl_xor_sync(0xffffffffu, l[n], 1);
+        l[n] += __shfl_xor_sync(0xffffffffu, l[n], 2);
+        float* p0 = part + (n * 8 + 2 * t) * (HD + 2);
+        float* p1 = p0 + (HD + 2);
+#pragma unroll
+        for (int j = 0; j < KS; ++j) {
+            const int da = (j >> 3) * 128 + g * 8 + (j & 7), db = da + 64;
+            p0[da] = o[n][j][0]; p1[da] = o[n][j][1];
+            p0[db] = o[n][j][2]; p1[db] = o[n][j][3];
+        }
+        if (t == 0) {
+            float* pg = part + (n * 8 + g) * (HD + 2);
+            pg[HD] = mx[n];
+            pg[HD + 1] = l[n];
+        }
+    }
+    __syncthreads();
+    constexpr int RS = D * kTileStage / 4;                                                        // floats between two rings
+    auto row_part = [&](int r) { return reinterpret_cast<const float*>(stream_smem + (r / RW) * kTileStage) + (r % RW) * (HD + 2); };
+    float* ring_w = reinterpret_cast<float*>(k_s + a.M * 32);                                     // [rows][NR] weight of each ring's partial
+    const size_t w0 = (static_cast<size_t>(kv) * a.n_splits + blockIdx.x) * rows_all + r0;
+    if (static_cast<int>(threadIdx.x) < rows) {
+        const float* p0 = row_part(threadIdx.x);
+        float M_ = -INFINITY, L_ = 0.f;
+#pragma unroll
+        for (int q = 0; q < NR; ++q) M_ = fmaxf(M_, p0[q * RS + HD]);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const float w = p0[q * RS + HD] == -INFINITY ? 0.f : exp2f(p0[q * RS + HD] - M_);
+            ring_w[threadIdx.x * NR + q] = w;
+            L_ = fmaf(p0[q * RS + HD + 1], w, L_);
+        }
+        *reinterpret_cast<float2*>(a.ws_ml + (w0 + threadIdx.x) * 2) = make_float2(M_, L_);
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < rows * HD / 2; idx += blockDim.x) {                         // the rows of a partial are 8-byte aligned
+        const int r = idx / (HD / 2), d = idx % (HD / 2) * 2;
+        const float* p0 = row_part(r) + d;
+        float2 A_ = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            const float w = ring_w[r * NR + q];
+            const float2 x = *reinterpret_cast<const float2*>(p0 + q * RS);
+            A_.x = fmaf(x.x, w, A_.x); A_.y = fmaf(x.y, w, A_.y);
+        }
+        *reinterpret_cast<float2*>(a.ws_acc + (w0 + r) * HD + d) = A_;
+    }
+    tr.mark(3);
+}
+
+// One CTA per (row, kv head, 64 dims): adds the CTAs' partials, gates and stores.  Sixteen groups of 64 threads take every 16th
+// partial, so that all of them are requested at once.
+constexpr int kMergeDims = 64;
+__global__ void __launch_bounds__(1024) attn_merge_kernel(AttnDecodeArgs a, int min_keys, int grid_x, int rings) {
+    constexpr int HD = kStreamHd, GROUPS = 1024 / kMergeDims, WAY = 160 / GROUPS;
+    __shared__ float s_w[160], s_l, s_acc[GROUPS][kMergeDims];
+    TraceCta tr;
+    tr.begin(kTrHelper);
+    pdl_launch_dependents();
+    const int row = blockIdx.x, kv = blockIdx.y, G = a.nq / a.kvh, rows_all = a.M * G, q = threadIdx.x / kMergeDims, dl = threadIdx.x % kMergeDims,
+              d = blockIdx.z * kMergeDims + dl, m = row / G;
+    int C0 = 0;
+    if (a.flags & 8) C0 = *reinterpret_cast<const volatile int*>(a.ctl + kCtlCommittedLen);
+    pdl_wait();
+    tr.mark(1);
+    if (!(a.flags & 8)) C0 = a.ctl[kCtlCommittedLen];
+    const int n_keys = min(C0 + a.M, a.cache_len);
+    if (n_keys <= min_keys) { tr.mark(3); return; }
+    const size_t o = (static_cast<size_t>(m) * a.ngate + kv * G + row % G) * HD + d;
+    const float gate = q == 0 ? __ldcg(a.gate + o) : 0.f;
+    // the ranges of attn_stream_kernel: CTAs past the last key have stored nothing
+    const int n_act = max(1, min(grid_x, (n_keys + rings * kTileKeys - 1) / (rings * kTileKeys)));
+    const int tiles = (n_keys + kTileKeys - 1) / kTileKeys, per = (tiles + n_act - 1) / n_act, n = (tiles + per - 1) / per;
+    const size_t w0 = static_cast<size_t>(kv) * a.n_splits * rows_all + row;
+    float v[WAY];
+#pragma unroll
+    for (int i = 0; i < WAY; ++i) {
+        const int c = q + GROUPS * i;
+        v[i] = c < n ? __ldcg(a.ws_acc + (w0 + static_cast<size_t>(c) * rows_all) * HD + d) : 0.f;
+    }
+    if (threadIdx.x < 32) {
+        float ml[5], ll[5], mxv = -INFINITY, sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const int c = static_cast<int>(threadIdx.x) + 32 * i;
+            const float2 x = c < n ? __ldcg(reinterpret_cast<const float2*>(a.ws_ml) + w0 + static_cast<size_t>(c) * rows_all) : make_float2(-INFINITY, 0.f);
+            ml[i] = x.x; ll[i] = x.y;
+            mxv = fmaxf(mxv, x.x);
+        }
+        mxv = warp_max(mxv);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const float w = ml[i] == -INFINITY ? 0.f : exp2f(ml[i] - mxv);
+            s_w[threadIdx.x + 32 * i] = w;
+            sum = fmaf(ll[i], w, sum);
+        }
+        sum = warp_sum(sum);
+        if (threadIdx.x == 0) s_l = sum;
+    }
+    __syncthreads();
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < WAY; ++i) {
+        const int c = q + GROUPS * i;
+        if (c < n) acc = fmaf(v[i], s_w[c], acc);
+    }
+    s_acc[q][dl] = acc;
+    __syncthreads();
+    if (q == 0) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < GROUPS; ++i) sum += s_acc[i][dl];
+        a.out[o] = (s_l > 0.f ? sum / s_l : 0.f) * sigmoid_f(gate);
+    }
+    tr.mark(3);
+}
+
 }  // namespace nexrt
 
 using namespace nexrt;
@@ -1037,6 +1437,65 @@ extern "C" size_t nexrt_attn_decode_smem(int hd, int nq, int kvh, int M) {
     return sizeof(float) * (main_floats > combine_floats ? main_floats : combine_floats);
 }
 
+// Launches the cluster kernel; with more than max_keys keys in its window it does nothing.
+static int launch_cluster_form(const AttnDecodeArgs& a, int hd, int kvh, int n_splits, int max_keys, cudaStream_t st) {
+    // cluster form: whole clusters along x; its shared memory adds this CTA's partial for the DSMEM combine
+    const int passes_c = (a.M * (a.nq / kvh) + kRowsPerPassMma - 1) / kRowsPerPassMma;
+    const size_t rows = static_cast<size_t>(a.M) * (a.nq / kvh);
+    const size_t smem_c = sizeof(float) * (rows * hd + static_cast<size_t>(a.M) * hd + 8 * kRowsPerPassMma * (hd + 2) + static_cast<size_t>(hd / 16) * 32 * 4 +
+                                           kRowsPerPassMma * hd + kRowsPerPassMma * 2);
+    const size_t smem_max = sizeof(float) * (static_cast<size_t>(kMaxRows) * (a.nq / kvh) * hd + static_cast<size_t>(kMaxRows) * hd +
+                                             8 * kRowsPerPassMma * (hd + 2) + static_cast<size_t>(hd / 16) * 32 * 4 + kRowsPerPassMma * hd + kRowsPerPassMma * 2);
+    // clusters of 16 (non-portable size) when asked for and when the device can place one: twice the warps per cluster, so a
+    // context of up to 2048 keys is one 16-key tile per warp and still needs no cross-cluster tail
+    const int groups = kvh * passes_c;                      // cluster rows of the grid (y x z)
+    if ((gemv_mode() & 128) && n_splits >= kClusterCtasWide) {
+        const int cap = hd == 256 ? cluster_capacity<256, kClusterCtasWide>(smem_max) : (hd == 128 ? cluster_capacity<128, kClusterCtasWide>(smem_max) : 0);
+        if (cap > 0) {
+            const int n_clusters = max(1, min(n_splits / kClusterCtasWide, cap / groups));
+            const dim3 gw(n_clusters * kClusterCtasWide, kvh, passes_c);
+            if (hd == 256) return launch_cluster(attn_decode_cluster_kernel<256, kClusterCtasWide>, gw, dim3(256), smem_c, st, kClusterCtasWide, a, max_keys);
+            return launch_cluster(attn_decode_cluster_kernel<128, kClusterCtasWide>, gw, dim3(256), smem_c, st, kClusterCtasWide, a, max_keys);
+        }
+    }
+    const int cap8 = hd == 256 ? cluster_capacity<256, kClusterCtas>(smem_max) : (hd == 128 ? cluster_capacity<128, kClusterCtas>(smem_max) : 0);
+    const int n_clusters = max(1, min(n_splits / kClusterCtas, cap8 > 0 ? cap8 / groups : n_splits / kClusterCtas));
+    const dim3 g(n_clusters * kClusterCtas, kvh, passes_c);
+    if (hd == 256) return launch_cluster(attn_decode_cluster_kernel<256, kClusterCtas>, g, dim3(256), smem_c, st, kClusterCtas, a, max_keys);
+    if (hd == 128) return launch_cluster(attn_decode_cluster_kernel<128, kClusterCtas>, g, dim3(256), smem_c, st, kClusterCtas, a, max_keys);
+    return cudaErrorInvalidValue;
+}
+
+// Context length from which the streaming form works instead of the cluster kernel (INT_MAX: never).  It exists for head dim 256
+// and plain causal windows; context-parallel groups, sliding windows, non-causal and ungated blocks stay on the cluster kernel.
+// The lines, us a layer, cluster kernel / streaming form (B200):
+//   one kv head, up to seven passes of eight rows: up to 2048 keys the cluster kernel has one tile per warp.  One row of four
+//     heads 20.2 / 21.7 at 1100 keys, 27.0 / 22.3 at 4200; eight rows 30.3 / 38.2 and 36.8 / 36.8 (31.5 with the shorter prologue).
+//   two kv heads, one row of 16 heads each: 51.4 / 54 at 4200, 57.4 / 55.3 at 8400.
+//   from eight passes up the cluster kernel's clusters no longer fit the device together: four rows of 2 x 16 heads 101 / 72 at 64
+//     keys, 174 / 95 at 16800; eight rows 184 / 84 and 300 / 126.
+static int stream_min_keys(const AttnDecodeArgs& a, int hd, int cp_size, int window) {
+    if (hd != kStreamHd || cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate || a.rotary > hd) return INT_MAX;
+    const int rows = a.M * (a.nq / a.kvh);
+    const size_t smem = rows <= 8 ? attn_stream_smem<1, 1>(a.M, a.rotary) : (rows <= 16 ? attn_stream_smem<2, 1>(a.M, a.rotary) : attn_stream_smem<2, 2>(a.M, a.rotary));
+    if (smem > 227 * 1024) return INT_MAX;
+    const int passes = a.kvh * ((rows + kRowsPerPassMma - 1) / kRowsPerPassMma);
+    return passes >= 8 ? 0 : (a.kvh == 1 ? kStreamFrom : kStreamFromTwoHeads);
+}
+
+template <int NTR, int WR>
+static int launch_stream(const AttnDecodeArgs& a, int min_keys, cudaStream_t st) {
+    const int rows = a.M * (a.nq / a.kvh), passes = (rows + 8 * NTR * WR - 1) / (8 * NTR * WR);
+    const int splits = max(1, min(min(a.n_splits, 160), sm_count() / (a.kvh * passes)));
+    if (const int e = launch(attn_stream_kernel<NTR, WR>, dim3(splits, a.kvh, passes), dim3(stream_rings<WR>() * WR * 32), attn_stream_smem<NTR, WR>(a.M, a.rotary), st, a, min_keys))
+        return e;
+    return launch(attn_merge_kernel, dim3(rows, a.kvh, kStreamHd / kMergeDims), dim3(1024), 0, st, a, min_keys, splits, stream_rings<WR>());
+}
+static int launch_stream_form(const AttnDecodeArgs& a, int min_keys, cudaStream_t st) {
+    const int rows = a.M * (a.nq / a.kvh);
+    return rows <= 8 ? launch_stream<1, 1>(a, min_keys, st) : (rows <= 16 ? launch_stream<2, 1>(a, min_keys, st) : launch_stream<2, 2>(a, min_keys, st));
+}
+
 extern "C" int nexrt_attn_decode(const void* q_raw, const void* gate, const void* k_raw, const void* qn, const void* kn, const void* inv_freq,
                                  const void* rope_table, const void* ctl, void* k_cache, const void* v_cache, void* ws_acc, void* ws_ml, void* ticket, void* out,
                                  int hd, int nq, int ngate, int kvh, int M, int cache_len, int rotary, int n_splits, float eps, int flags,
@@ -1060,31 +1519,10 @@ extern "C" int nexrt_attn_decode(const void* q_raw, const void* gate, const void
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool mma = (gemv_mode() & 32) != 0;
     if (mma && (gemv_mode() & 64) && n_splits >= kClusterCtas) {
-        // cluster form: whole clusters along x; its shared memory adds this CTA's partial for the DSMEM combine
-        const int passes_c = (M * (nq / kvh) + kRowsPerPassMma - 1) / kRowsPerPassMma;
-        const size_t rows = static_cast<size_t>(M) * (nq / kvh);
-        const size_t smem_c = sizeof(float) * (rows * hd + static_cast<size_t>(M) * hd + 8 * kRowsPerPassMma * (hd + 2) + static_cast<size_t>(hd / 16) * 32 * 4 +
-                                               kRowsPerPassMma * hd + kRowsPerPassMma * 2);
-        const size_t smem_max = sizeof(float) * (static_cast<size_t>(kMaxRows) * (nq / kvh) * hd + static_cast<size_t>(kMaxRows) * hd +
-                                                 8 * kRowsPerPassMma * (hd + 2) + static_cast<size_t>(hd / 16) * 32 * 4 + kRowsPerPassMma * hd + kRowsPerPassMma * 2);
-        // clusters of 16 (non-portable size) when asked for and when the device can place one: twice the warps per cluster, so a
-        // context of up to 2048 keys is one 16-key tile per warp and still needs no cross-cluster tail
-        const int groups = kvh * passes_c;                      // cluster rows of the grid (y x z)
-        if ((gemv_mode() & 128) && n_splits >= kClusterCtasWide) {
-            const int cap = hd == 256 ? cluster_capacity<256, kClusterCtasWide>(smem_max) : (hd == 128 ? cluster_capacity<128, kClusterCtasWide>(smem_max) : 0);
-            if (cap > 0) {
-                const int n_clusters = max(1, min(n_splits / kClusterCtasWide, cap / groups));
-                const dim3 gw(n_clusters * kClusterCtasWide, kvh, passes_c);
-                if (hd == 256) return launch_cluster(attn_decode_cluster_kernel<256, kClusterCtasWide>, gw, dim3(256), smem_c, st, kClusterCtasWide, a);
-                return launch_cluster(attn_decode_cluster_kernel<128, kClusterCtasWide>, gw, dim3(256), smem_c, st, kClusterCtasWide, a);
-            }
-        }
-        const int cap8 = hd == 256 ? cluster_capacity<256, kClusterCtas>(smem_max) : (hd == 128 ? cluster_capacity<128, kClusterCtas>(smem_max) : 0);
-        const int n_clusters = max(1, min(n_splits / kClusterCtas, cap8 > 0 ? cap8 / groups : n_splits / kClusterCtas));
-        const dim3 g(n_clusters * kClusterCtas, kvh, passes_c);
-        if (hd == 256) return launch_cluster(attn_decode_cluster_kernel<256, kClusterCtas>, g, dim3(256), smem_c, st, kClusterCtas, a);
-        if (hd == 128) return launch_cluster(attn_decode_cluster_kernel<128, kClusterCtas>, g, dim3(256), smem_c, st, kClusterCtas, a);
-        return cudaErrorInvalidValue;
+        const int stream_from = stream_min_keys(a, hd, cp_size, window);
+        if (stream_from > 0)
+            if (const int e = launch_cluster_form(a, hd, kvh, n_splits, stream_from, st)) return e;
+        return a.cache_len > stream_from ? launch_stream_form(a, stream_from, st) : 0;
     }
     a.flags &= ~8;   // only the cluster kernel reads the control block before its dependency wait
     const int passes = (M * (nq / kvh) + kRowsPerPassMma - 1) / kRowsPerPassMma;     // tensor-core path: eight query rows per CTA

@@ -125,18 +125,19 @@ __device__ __forceinline__ void attn_mma_pass(const AttnMmaKeys& k, const uint4*
         prefetch_rows(k.vc, tile, k.hi);
         prefetch_rows(k.kc, tile + 16 * nwarps, min(k.hi, k.C0));
         // ---- scores of 16 keys: tile + g (s0) and tile + 8 + g (s1) on the N side
-        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+        // (hi and lo products in accumulators of their own: a lo product on the hi product's accumulator would wait for it)
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, z0[4] = {0.f, 0.f, 0.f, 0.f}, z1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
             const uint4 q = qf[ks * 32 + lane];
             const int b = ks >> 2, s = ks & 3;
             mma_bf16_16x8x16(s0, q.x, 0u, q.y, 0u, ka[b][2 * s], ka[b][2 * s + 1]);
-            if (EXACT) mma_bf16_16x8x16(s0, q.z, 0u, q.w, 0u, ka[b][2 * s], ka[b][2 * s + 1]);
+            if (EXACT) mma_bf16_16x8x16(z0, q.z, 0u, q.w, 0u, ka[b][2 * s], ka[b][2 * s + 1]);
             mma_bf16_16x8x16(s1, q.x, 0u, q.y, 0u, kb[b][2 * s], kb[b][2 * s + 1]);
-            if (EXACT) mma_bf16_16x8x16(s1, q.z, 0u, q.w, 0u, kb[b][2 * s], kb[b][2 * s + 1]);
+            if (EXACT) mma_bf16_16x8x16(z1, q.z, 0u, q.w, 0u, kb[b][2 * s], kb[b][2 * s + 1]);
         }
         // ---- mask and online softmax of row g (its 16 scores sit in the 4 lanes that share g)
-        float sv[4] = {s0[0], s0[1], s1[0], s1[1]};
+        float sv[4] = {s0[0] + z0[0], s0[1] + z0[1], s1[0] + z1[0], s1[1] + z1[1]};
         const int kp[4] = {tile + 2 * t, tile + 2 * t + 1, tile + 8 + 2 * t, tile + 9 + 2 * t};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -176,14 +177,23 @@ __device__ __forceinline__ void attn_mma_pass(const AttnMmaKeys& k, const uint4*
                     v[i][0] = v[i][1] = make_uint4(0u, 0u, 0u, 0u);
                 }
             }
+            // hi products of two output tiles, then their lo products (issued in the order written, see above)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
-                auto word = [&](const uint4& q4) { return (j >> 1) == 0 ? q4.x : ((j >> 1) == 1 ? q4.y : ((j >> 1) == 2 ? q4.z : q4.w)); };
-                const uint32_t a0 = prmt(word(v[0][0]), word(v[1][0]), sel), a1 = prmt(word(v[0][1]), word(v[1][1]), sel);
-                const uint32_t a2 = prmt(word(v[2][0]), word(v[3][0]), sel), a3 = prmt(word(v[2][1]), word(v[3][1]), sel);
-                mma_bf16_16x8x16(o[blk * 8 + j], a0, a1, a2, a3, ph0, ph1);
-                if (EXACT) mma_bf16_16x8x16(o[blk * 8 + j], a0, a1, a2, a3, pl0, pl1);
+            for (int j0 = 0; j0 < 8; j0 += 2) {
+                uint32_t av[2][4];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int j = j0 + u;
+                    const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+                    auto word = [&](const uint4& q4) { return (j >> 1) == 0 ? q4.x : ((j >> 1) == 1 ? q4.y : ((j >> 1) == 2 ? q4.z : q4.w)); };
+                    av[u][0] = prmt(word(v[0][0]), word(v[1][0]), sel); av[u][1] = prmt(word(v[0][1]), word(v[1][1]), sel);
+                    av[u][2] = prmt(word(v[2][0]), word(v[3][0]), sel); av[u][3] = prmt(word(v[2][1]), word(v[3][1]), sel);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) mma_bf16_16x8x16(o[blk * 8 + j0 + u], av[u][0], av[u][1], av[u][2], av[u][3], ph0, ph1);
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (EXACT) mma_bf16_16x8x16(o[blk * 8 + j0 + u], av[u][0], av[u][1], av[u][2], av[u][3], pl0, pl1);
             }
         }
     }

@@ -1,0 +1,58 @@
+"""Decode attention with a cache long enough for the streaming form, against float64: contexts on both sides of the line where it
+takes over, at the edges of its 16-key tiles, with fewer tiles than rings and more, one to several row groups and passes."""
+
+import pytest
+import torch
+
+from nexrt_b200.ops.lib import check, load, ptr
+from nexrt_b200.runtime.control import CTL_WORDS, Ctl
+
+pytestmark = pytest.mark.gpu
+DEV, HD, ROT = "cuda", 256, 64
+
+
+@pytest.mark.parametrize("M,nq,kvh", [(1, 4, 1), (2, 4, 1), (3, 4, 1), (8, 4, 1), (1, 8, 1), (5, 8, 1), (1, 32, 2), (8, 32, 2), (8, 8, 4)])
+@pytest.mark.parametrize("C0", [5, 1023, 1040, 1301, 4095, 4097, 9999, 20000])
+def test_long_context_decode(M, nq, kvh, C0):
+    g = torch.Generator(device=DEV).manual_seed(M * 1000 + nq + C0)
+    cache, n_splits, G = max(C0, 6000) + M + 3, 148 // kvh, nq // kvh
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, gate, k, qn, kn = rn(8, nq, HD), rn(8, nq, HD), rn(8, kvh, HD), 1 + 0.1 * rn(HD), 1 + 0.1 * rn(HD)
+    kc, vc = rn(kvh, cache, HD).to(torch.bfloat16), rn(kvh, cache, HD).to(torch.bfloat16)
+    kc[:, C0:] = float("nan")                                  # rows of the future: never read
+    vc[:, C0 + M :] = float("nan")
+    inv = 1.0 / (1e7 ** (torch.arange(0, ROT, 2, dtype=torch.float32) / ROT)).to(DEV)
+    ang = torch.arange(cache, dtype=torch.float32, device=DEV)[:, None] * inv[None, :]
+    rope = torch.stack([ang.cos(), ang.sin()], -1).contiguous()
+    ctl = torch.zeros(CTL_WORDS, dtype=torch.int32, device=DEV)
+    ctl[Ctl.COMMITTED_LEN] = C0
+    ws_acc, ws_ml = torch.full((kvh, n_splits, 8 * G, HD), float("nan"), device=DEV), torch.full((kvh, n_splits, 8 * G, 2), float("nan"), device=DEV)
+    ticket, out = torch.zeros(kvh, dtype=torch.int32, device=DEV), torch.zeros(8, nq * HD, device=DEV)
+    for flags in (8, 0):
+        out.zero_()
+        kcc = kc.clone()
+        check(load().nexrt_attn_decode(ptr(q), ptr(gate), ptr(k), ptr(qn), ptr(kn), ptr(inv), ptr(rope), ptr(ctl), ptr(kcc), ptr(vc), ptr(ws_acc), ptr(ws_ml), ptr(ticket),
+                                       ptr(out), HD, nq, nq, kvh, M, cache, ROT, n_splits, 1e-6, flags, 0, 0, 0, 1, 0, None, 0,
+                                       torch.cuda.current_stream().cuda_stream), "attn_decode")
+        torch.cuda.synchronize()
+        norm = lambda x, w: x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+
+        def rot(x):
+            c, s = rope[C0 : C0 + M, :, 0].double()[:, None], rope[C0 : C0 + M, :, 1].double()[:, None]
+            a, b = x[..., : ROT // 2], x[..., ROT // 2 : ROT]
+            return torch.cat([a * c - b * s, b * c + a * s, x[..., ROT:]], -1)
+
+        qd, kd = rot(norm(q[:M].double(), qn)), rot(norm(k[:M].double(), kn))
+        new = kcc[:, C0 : C0 + M].double()
+        assert ((new - kd.transpose(0, 1)).abs() <= 2.0**-8 * kd.transpose(0, 1).abs() + 1e-5).all()
+        assert torch.equal(kcc[:, :C0], kc[:, :C0])
+        K, V = torch.cat([kc[:, :C0].double(), new], 1), vc[:, : C0 + M].double()
+        sc = torch.einsum("mhgd,hkd->mhgk", qd.view(M, kvh, G, HD), K) / 16.0
+        sc = sc.masked_fill(torch.arange(C0 + M, device=DEV) > torch.arange(C0, C0 + M, device=DEV)[:, None, None, None], -float("inf"))
+        p = torch.softmax(sc, -1)
+        ctx = torch.einsum("mhgk,hkd->mhgd", p, V).reshape(M, nq, HD) * torch.sigmoid(gate[:M].double())
+        # Q and P are bf16 hi + lo (2^-17), everything else fp32: errors stay below 2^-14 of sum p |v|
+        bound = 2.0**-14 * torch.einsum("mhgk,hkd->mhgd", p, V.abs()).reshape(M, nq, HD) + 1e-6
+        err = (out[:M].view(M, nq, HD).double() - ctx).abs()
+        assert (err <= bound).all(), (err / bound).max()
+        assert not out[M:].any()
