@@ -187,6 +187,8 @@ int nexrt_attn_front_rows(const void* x, const void* in_ln, const void* w, const
 
 int nexrt_tc_router_logits(const void* x, const void* gamma, const void* w, void* planes, void* partial, const void* zero_ids, int rows, int rows_pad, int K,
                            int M, int ksplit, float eps, void* planes_e4m3, int* status, void* stream);   /* partial: [ksplit][M][rows_pad] */
+int nexrt_moe_router_rows(const void* x, const void* post_ln, const void* w, void* cols, void* partial, void* planes_e4m3, int rows_pad, int H, int M, float eps,
+                          void* stream);   /* 2..8 rows; cols: bf16 [2 M][H] scratch, partial: [4][M][rows_pad] */
 int nexrt_moe_router_topk(const void* partial, int ksplit, int rows_pad, void* logits, void* ids, void* wts, int E, int topk, int M, void* stream);
 
 int nexrt_lmhead_sample_from_logits(const void* logits_in, void* cand, void* ticket, const void* sampling, void* ctl, void* export_buf, int H, int V_local,

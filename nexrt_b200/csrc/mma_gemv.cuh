@@ -545,15 +545,16 @@ struct MmaStream {
 constexpr int kStreamWarps = 8;
 constexpr int kStreamPad = 64;      // bytes behind each activation column (see MmaStream::group)
 
-// Asynchronous copy of the step's activation columns ([ncols][col_bytes] in global memory, col_bytes a multiple of 16) into
-// shared memory columns ldx bytes apart; complete for this thread on return.  One warp per column, and every CTA starts at another place: all CTAs read
+// Asynchronous copy of the step's activation columns (col_bytes, a multiple of 16, of each of ncols columns: from byte src_off
+// on of columns src_stride bytes apart; src_stride 0: packed) into shared memory columns ldx bytes apart; complete for this thread on return.  One warp per column, and every CTA starts at another place: all CTAs read
 // the same lines, and in the same order they would queue at one L2 slice after the other.
-__device__ __forceinline__ void stage_columns(uint8_t* xq, int ldx, const uint8_t* planes, int ncols, int col_bytes) {
+__device__ __forceinline__ void stage_columns(uint8_t* xq, int ldx, const uint8_t* planes, int ncols, int col_bytes, size_t src_stride = 0,
+                                              size_t src_off = 0) {
     const int pieces = col_bytes / 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int rot = static_cast<int>(blockIdx.x * 37u % static_cast<unsigned int>(pieces));
     for (int j = warp; j < ncols; j += nw) {
         const int col = (j + static_cast<int>(blockIdx.x)) % ncols;
-        const uint8_t* src = planes + static_cast<size_t>(col) * col_bytes;
+        const uint8_t* src = planes + static_cast<size_t>(col) * (src_stride ? src_stride : col_bytes) + src_off;
         const unsigned int dst = static_cast<unsigned int>(__cvta_generic_to_shared(xq + static_cast<size_t>(col) * ldx));
         for (int c0 = lane; c0 < pieces; c0 += 32) {
             const int c = c0 + rot < pieces ? c0 + rot : c0 + rot - pieces;

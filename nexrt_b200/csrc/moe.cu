@@ -25,6 +25,8 @@
 
 #include <atomic>
 
+int launch_rows_norm_split_bf16(const void* x, const void* gamma, void* planes, void* planes_e4m3, int K, int M, float eps, cudaStream_t st);   // tc_moe.cu
+
 namespace nexrt {
 
 // ---------------------------------------------------------------------------------------------
@@ -436,6 +438,73 @@ __global__ void __launch_bounds__(256, 2) moe_router_mma_kernel(RouterArgs a) {
     tr.mark(3);
 }
 
+// Router of several rows: the rows come normalised as bf16 hi and lo columns (cols [2 M][H], written by the kernel in front
+// together with the experts' e4m3 terms), one CTA takes 16 router rows and a quarter of H, and its eight warps hold their
+// weights in registers before the dependency wait.  The partial logits [4][M][rows_pad] are added by the top-k kernel.
+// One B200, 512 experts: the tcgen05 GEMM over K-split partials took 6.5 us at 8 rows, the one-row kernel's multi-row form,
+// which normalises and splits all rows in every CTA, 9.8 us at 4; here 3.8 us at 8 rows and 3.0 at 4 (behind 3.8 and 3.6 us for the rows).
+constexpr int kRouterRowsSplit = 4;
+template <int NT>
+__global__ void __launch_bounds__(256, 2) moe_router_rows_kernel(const __nv_bfloat16* __restrict__ w, const uint8_t* __restrict__ cols, float* __restrict__ partial, int H,
+                                                                 int M, int rows_pad) {
+    constexpr int KQ = kRouterRowsSplit, NB = 4, LD = 8 * NT + 1;     // NB windows of 64 bytes per warp: H <= 4096
+    extern __shared__ __align__(16) float smem[];
+    TraceCta tr;
+    tr.begin(kTrRouter);
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int row0 = (blockIdx.x / KQ) * kRowsPerGroup, kq = blockIdx.x % KQ, Kq = H / KQ, nwin = Kq / 32, ldx = 2 * Kq + kF16Pad;
+    float* tiles = smem;                                              // [8 warps][16][LD]
+    uint8_t* xq = reinterpret_cast<uint8_t*>(tiles + 8 * 16 * LD);    // [2 M][ldx]
+    xq += (16 - (reinterpret_cast<uintptr_t>(xq) & 15)) & 15;
+    uint4 ra[NB], rb[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int win = warp + 8 * i;
+        ra[i] = rb[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (win < nwin) {
+            const __nv_bfloat16* p = w + static_cast<size_t>(row0 + g) * H + kq * Kq + win * 32 + t * 8;
+            ra[i] = ld_stream16(p);
+            rb[i] = ld_stream16(p + static_cast<size_t>(8) * H);
+        }
+    }
+    pdl_wait();
+    tr.mark(1);
+    stage_columns(xq, ldx, cols, 2 * M, 2 * Kq, static_cast<size_t>(2) * H, static_cast<size_t>(2) * Kq * kq);
+    __syncthreads();
+    float d[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int win = warp + 8 * i;
+        if (win < nwin) {                                             // uniform across the warp
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                uint4 xb = make_uint4(0u, 0u, 0u, 0u);
+                if (nt * 8 + g < 2 * M) xb = *reinterpret_cast<const uint4*>(xq + static_cast<size_t>(nt * 8 + g) * ldx + win * 64 + t * 16);
+                mma_bf16_16x8x16(d[nt], ra[i].x, rb[i].x, ra[i].y, rb[i].y, xb.x, xb.y);
+                mma_bf16_16x8x16(d[nt], ra[i].z, rb[i].z, ra[i].w, rb[i].w, xb.z, xb.w);
+            }
+        }
+    }
+    float* tile = tiles + warp * 16 * LD;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        tile[g * LD + nt * 8 + 2 * t] = d[nt][0]; tile[g * LD + nt * 8 + 2 * t + 1] = d[nt][1];
+        tile[(g + 8) * LD + nt * 8 + 2 * t] = d[nt][2]; tile[(g + 8) * LD + nt * 8 + 2 * t + 1] = d[nt][3];
+    }
+    __syncthreads();
+    const int r = threadIdx.x % kRowsPerGroup, m = threadIdx.x / kRowsPerGroup;
+    if (m < M) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v += tiles[(k * 16 + r) * LD + 2 * m] + tiles[(k * 16 + r) * LD + 2 * m + 1];
+        partial[(static_cast<size_t>(kq) * M + m) * rows_pad + row0 + r] = v;
+    }
+    tr.mark(3);
+}
+
 // Top-k stage of the wide router (multi-row steps): the logits arrive as K-split partial planes
 // partial[ks][m][rows_pad] from the tcgen05 rows GEMM; they are added in a fixed order into shared memory, kept
 // in a.logits for inspection, and selected exactly like the fused router does.
@@ -675,6 +744,24 @@ extern "C" int nexrt_moe_router(const void* x, const void* post_ln, const void* 
     const size_t smem = sizeof(float) * (static_cast<size_t>(mb + 1) * H + gemv_part_floats((E + 1 + n_cta - 1) / n_cta, mb, gemv_geom(H / 8, gemv_threads())));
     if (M == 1) return launch(moe_router_kernel<1>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
     return launch(moe_router_kernel<4>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
+}
+
+// Partial router logits of 2..8 rows (partial: [4][M][rows_pad], for nexrt_moe_router_topk with ksplit 4) and the experts' terms
+// planes_e4m3 [3 M][H]; cols: bf16 [2 M][H] scratch.  cudaErrorNotSupported, with nothing launched, for shapes outside this form.
+extern "C" int nexrt_moe_router_rows(const void* x, const void* post_ln, const void* w, void* cols, void* partial, void* planes_e4m3, int rows_pad, int H, int M,
+                                     float eps, void* stream) {
+    if (M < 1 || M > kMaxRows || rows_pad < 1) return cudaErrorInvalidValue;
+    if (!(gemv_mode() & 16) || rows_pad % 16 || H % (32 * kRouterRowsSplit) || H > 4096) return cudaErrorNotSupported;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (const int e = launch_rows_norm_split_bf16(x, post_ln, cols, planes_e4m3, H, M, eps, st)) return e;
+    const int nt = (2 * M + 7) / 8;
+    const size_t smem = sizeof(float) * 8 * 16 * (8 * nt + 1) + static_cast<size_t>(2 * M) * (2 * (H / kRouterRowsSplit) + kF16Pad) + 16;
+    const dim3 grid(rows_pad / kRowsPerGroup * kRouterRowsSplit), block(256);
+    const __nv_bfloat16* wp = static_cast<const __nv_bfloat16*>(w);
+    const uint8_t* cp = static_cast<const uint8_t*>(cols);
+    float* out = static_cast<float*>(partial);
+    return nt == 1 ? launch(moe_router_rows_kernel<1>, grid, block, smem, st, wp, cp, out, H, M, rows_pad)
+                   : launch(moe_router_rows_kernel<2>, grid, block, smem, st, wp, cp, out, H, M, rows_pad);
 }
 
 extern "C" int nexrt_moe_router_topk(const void* partial, int ksplit, int rows_pad, void* logits, void* ids, void* wts, int E, int topk, int M, void* stream) {

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_moe_kernel(const __grid_consta
     constexpr int NAB = 8;               // accumulator buffers in tensor memory
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_user[kMaxRows];     // gate/up: slot of row m that uses this CTA's expert, or -1
+    __shared__ int s_ids[kMaxRows * 16];  // the step's expert ids [M][S]: one load for all of them (walked in global memory, the plan was the longest part of the prologue)
     __shared__ float s_wscale[kMaxKBlocks + 16 * 8];   // block scale of every K block this CTA walks (no load in the loop)
     TraceCta tr;
     tr.begin(a.trace_kind);
@@ -111,17 +112,17 @@ __global__ void __launch_bounds__(kThreads, 2) tc_moe_kernel(const __grid_consta
     pdl_wait();
     tr.mark(1);
     bool active = true;
+    if (static_cast<int>(threadIdx.x) < a.M * a.S) s_ids[threadIdx.x] = a.ids[threadIdx.x];
     if (!DOWN) {
+        __syncthreads();
         // route plan: the first row that names an expert computes it for every row that does
-        expert = a.ids[m * a.S + slot];
-        for (int m2 = 0; m2 < m; ++m2)
-            for (int s2 = 0; s2 < a.S; ++s2)
-                if (a.ids[m2 * a.S + s2] == expert) active = false;   // uniform for the CTA
+        expert = s_ids[m * a.S + slot];
+        active = __syncthreads_or(static_cast<int>(threadIdx.x) < m * a.S && s_ids[threadIdx.x] == expert) == 0;
         if (threadIdx.x < kMaxRows) {
             int u = -1;
             if (static_cast<int>(threadIdx.x) >= m && static_cast<int>(threadIdx.x) < a.M)
                 for (int s2 = 0; s2 < a.S; ++s2)
-                    if (a.ids[threadIdx.x * a.S + s2] == expert) u = s2;
+                    if (s_ids[threadIdx.x * a.S + s2] == expert) u = s2;
             s_user[threadIdx.x] = u;
         }
     }
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_moe_kernel(const __grid_consta
     const int n_kb = active ? KB : 0;
 
     // weight rows of K block kb start at this row of the flattened expert matrix
-    auto expert_of = [&](int kb) { return min(max(DOWN ? a.ids[m * a.S + kb / kpe] : expert, 0), a.n_total - 1); };   // kb: index in this CTA's range
+    auto expert_of = [&](int kb) { return min(max(DOWN ? s_ids[m * a.S + kb / kpe] : expert, 0), a.n_total - 1); };   // kb: index in this CTA's range
     const int rows_per_expert = DOWN ? a.H : I2;
 
     if (warp == 0) {
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(256) rows_norm_split_kernel(const __nv_bfloat1
 }
 
 // rmsnorm(x[m]) * gamma -> bf16 planes[(2m + {hi, lo})][H]: x' = hi + lo to ~2^-17
-__global__ void __launch_bounds__(256) rows_norm_split_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, __nv_bfloat16* planes,
+__global__ void __launch_bounds__(512) rows_norm_split_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, __nv_bfloat16* planes,
                                                                    uint8_t* planes_e4m3, int H, float eps) {
     __shared__ float red[32];
     extern __shared__ __align__(16) float xs[];
@@ -335,6 +336,12 @@ int launch_tc_moe(const CUtensorMap& mw, const CUtensorMap& mx, const TcMoeArgs&
 
 }  // namespace
 
+// rmsnorm(x[m]) * gamma of M rows -> bf16 hi and lo planes [2M][K] and, if planes_e4m3 != null, the e4m3 terms [3M][K].
+int launch_rows_norm_split_bf16(const void* x, const void* gamma, void* planes, void* planes_e4m3, int K, int M, float eps, cudaStream_t st) {
+    return launch(rows_norm_split_bf16_kernel, dim3(M), dim3(512), sizeof(float) * K, st, static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(gamma),
+                  static_cast<__nv_bfloat16*>(planes), static_cast<uint8_t*>(planes_e4m3), K, eps);
+}
+
 extern "C" {
 
 // Gate/up projections of all rows' experts.  planes: e4m3 [3M][H] scratch, written here.
@@ -364,8 +371,7 @@ int nexrt_tc_router_logits(const void* x, const void* gamma, const void* w, void
                            int M, int ksplit, float eps, void* planes_e4m3, int* status, void* stream) {
     if (M < 1 || M > kMaxRows || K % 64 || K > 4096 || rows_pad % 2 || rows_pad < rows || ksplit < 1 || ksplit > 16) return cudaErrorInvalidValue;
     auto st = static_cast<cudaStream_t>(stream);
-    int e = launch(rows_norm_split_bf16_kernel, dim3(M), dim3(256), sizeof(float) * K, st, static_cast<const __nv_bfloat16*>(x),
-                   static_cast<const float*>(gamma), static_cast<__nv_bfloat16*>(planes), static_cast<uint8_t*>(planes_e4m3), K, eps);
+    int e = launch_rows_norm_split_bf16(x, gamma, planes, planes_e4m3, K, M, eps, st);
     if (e) return e;
     CUtensorMap mw, mx;
     if (!tensor_map(&mw, w, rows, K, K, kBM, true) || !tensor_map(&mx, planes, 2 * M, K, K, kBN, true)) return cudaErrorInvalidValue;

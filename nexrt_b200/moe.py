@@ -15,7 +15,7 @@ import os
 
 import torch
 
-from .ops.lib import check, ptr
+from .ops.lib import NOT_SUPPORTED, check, ptr
 from .runtime.context import StepContext
 
 
@@ -30,7 +30,6 @@ class Moe:
             w["router_w_pad"] = pad
         # rows from which the experts run on the tcgen05 kernels (NEXRT_TC_MOE_ROWS=0 switches them off)
         self.tc_rows = int(os.environ.get("NEXRT_TC_MOE_ROWS", "2")) or 1 << 30
-        self.tc_router_rows = int(os.environ.get("NEXRT_TC_ROUTER_ROWS", "8")) or 1 << 30   # below 8 rows the fused router kernel is as fast
         cfg, spec = ctx.cfg, ctx.spec
         self.tc_ok = cfg.hidden % 128 == 0 and cfg.hidden <= 4096 and spec.inter % 128 == 0
         # the fused router takes its tensor-core form (the one that can also write the planes) under these conditions
@@ -46,35 +45,25 @@ class Moe:
 
     def forward(self, M: int = 1) -> None:
         c, w, lib = self.ctx, self.w, self.ctx.lib
-        cfg, spec, st = c.cfg, c.spec, c.stream()
-        S = cfg.top_k + 1
-        wide = M >= self.tc_router_rows and self.tc_ok and cfg.hidden % (64 * c.router_ksplit) == 0
+        cfg, st = c.cfg, c.stream()
         tc_experts = M >= self.tc_rows and self.tc_ok
-        # the routers of a step whose experts run on tcgen05 also leave the experts' activation planes
-        self._planes_ready = tc_experts and (wide or self.router_mma)
-        planes = ptr(c.moe_planes1) if self._planes_ready else None
-        if wide:
-            # multi-row steps: router logits of all rows in one tcgen05 GEMM (bf16 weights, hi + lo activation planes,
-            # K split over CTAs), then one small kernel adds the partial planes and selects the experts
-            check(
-                lib.nexrt_tc_router_logits(ptr(c.x), ptr(w["post_ln"]), ptr(w["router_w_pad"]), ptr(c.router_planes), ptr(c.router_partial), ptr(c.zero_ids),
-                                           cfg.n_experts + 1, self.rows_pad, cfg.hidden, M, c.router_ksplit, cfg.rms_eps, planes, ptr(c.status), st),
-                "tc_router_logits",
-            )
-            check(lib.nexrt_moe_router_topk(ptr(c.router_partial), c.router_ksplit, self.rows_pad, ptr(c.moe_logits), ptr(c.moe_ids), ptr(c.moe_wts),
-                                            cfg.n_experts, cfg.top_k, M, st), "moe_router_topk")
-        elif not tc_experts and self.routed_ok:
+        if not tc_experts and self.routed_ok:
             self._routed(M)
             return
-        elif self.routed_ok and self.router_mma:
-            # a few rows with the experts on tcgen05: the router stops at its partial logits (no ticket, no one-CTA tail)
-            # and a one-CTA node adds them and selects - two short nodes instead of one long one
-            check(lib.nexrt_moe_router_partial(ptr(c.x), ptr(w["post_ln"]), ptr(w["router_w_pad"]), ptr(c.moe_partial), self.rows_pad, cfg.hidden,
-                                               cfg.n_experts, cfg.top_k, M, cfg.rms_eps, planes, st), "moe_router_partial")
-            check(lib.nexrt_moe_router_topk(ptr(c.moe_partial), lib.nexrt_moe_router_partial_split(), self.rows_pad, ptr(c.moe_logits),
-                                            ptr(c.moe_ids), ptr(c.moe_wts), cfg.n_experts, cfg.top_k, M, st), "moe_router_topk")
+        # several rows: normalised once (as the router's columns and the experts' terms), the router's partial logits on all
+        # SMs, then one small kernel adds them and selects the experts
+        e = NOT_SUPPORTED
+        if tc_experts and M > 1:
+            e = lib.nexrt_moe_router_rows(ptr(c.x), ptr(w["post_ln"]), ptr(w["router_w_pad"]), ptr(c.router_planes), ptr(c.moe_partial), ptr(c.moe_planes1),
+                                          self.rows_pad, cfg.hidden, M, cfg.rms_eps, st)
+        if e == NOT_SUPPORTED:
+            self._planes_ready = tc_experts and self.router_mma
+            self._router_fused(M, ptr(c.moe_planes1) if self._planes_ready else None)
         else:
-            self._router_fused(M, planes)
+            check(e, "moe_router_rows")
+            self._planes_ready = True
+            check(lib.nexrt_moe_router_topk(ptr(c.moe_partial), 4, self.rows_pad, ptr(c.moe_logits), ptr(c.moe_ids), ptr(c.moe_wts), cfg.n_experts, cfg.top_k, M,
+                                            st), "moe_router_topk")
         self._experts(M)
 
     def _routed(self, M: int) -> None:

@@ -100,6 +100,7 @@ _PROTOTYPES = {
     "nexrt_gdn_front_rows": [vp] * 15 + [ci] * 6 + [cf, vp],
     "nexrt_attn_front_rows": [vp] * 10 + [ci] * 7 + [cf, vp],
     "nexrt_tc_router_logits": [vp] * 6 + [ci] * 5 + [cf, vp, vp, vp],
+    "nexrt_moe_router_rows": [vp] * 6 + [ci] * 3 + [cf, vp],
     "nexrt_moe_router_topk": [vp, ci, ci, vp, vp, vp, ci, ci, ci, vp],
     "nexrt_lmhead_sample_from_logits": [vp] * 6 + [ci] * 6 + [CH, cu, ci, vp],
     "nexrt_oproj_stage_split": [vp] * 5 + [ci, ci, ci, cf, ci, CH, cu, vp],

@@ -107,9 +107,7 @@ class StepContext:
         self.oproj_planes = z(3 * MAX_ROWS, max(spec.gdn_local, spec.attn_local), dtype=torch.uint8)
         self.oproj_descale = z(MAX_ROWS)
         self.tc_oproj_rows = int(os.environ.get("NEXRT_TC_OPROJ_ROWS", "0")) or 1 << 30   # measured no faster than the fused kernel at 4 and 8 rows: off unless asked for
-        self.router_ksplit = 8
         self.router_planes = z(2 * MAX_ROWS, cfg.hidden, dtype=torch.bfloat16)
-        self.router_partial = z(self.router_ksplit, MAX_ROWS, (cfg.n_experts + 1 + 15) // 16 * 16)
         # head scratch
         self.head_cand = z(MAX_ROWS, self.n_cta, MAX_TOPK, dtype=torch.int64)
         self.head_ticket = z(1, dtype=i32)
