@@ -102,8 +102,11 @@ __host__ __device__ inline GemvGeom gemv_geom(int chunks, int threads) {
     return g;
 }
 
-// shared-memory floats needed for the partials of `nrows` rows
-__host__ __device__ inline size_t gemv_part_floats(int nrows, int mb, const GemvGeom& g) { return static_cast<size_t>(nrows) * g.wpr * mb; }
+// shared-memory floats needed for the partials of `nrows` rows, rounded up to 16 bytes: what a kernel keeps behind them (norm
+// multipliers, keys) is read in wider pieces than one float
+__host__ __device__ inline size_t gemv_part_floats(int nrows, int mb, const GemvGeom& g) {
+    return (static_cast<size_t>(nrows) * g.wpr * mb + 3) / 4 * 4;
+}
 
 template <int EPL>
 __device__ __forceinline__ void unpack_chunk(const uint4& v, float* f) {
