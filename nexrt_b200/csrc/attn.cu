@@ -1342,7 +1342,7 @@ static int cluster_capacity(size_t smem) {
     if (cached >= 0) return cached;
     cached = 0;
     if (CL > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
+    if (opt_in_smem(kernel, smem) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }

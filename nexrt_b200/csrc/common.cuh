@@ -259,13 +259,17 @@ static inline int trace_install() {
 }
 #endif
 
+// Allows a kernel `smem` bytes of dynamic shared memory where the default may not.  The default limit of 48 KB counts static memory
+// too: no kernel that takes dynamic memory has more than 8 KB of it, so below 40 KB there is nothing to ask for.
+template <typename Kernel>
+static inline cudaError_t opt_in_smem(Kernel kernel, size_t smem) {
+    return smem > 40 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) : cudaSuccess;
+}
+
 template <typename... KArgs, typename... Args>
 static inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                   Args... args) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return static_cast<int>(e);
-    }
+    if (const cudaError_t e = opt_in_smem(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
 #ifdef NEXRT_TRACE
     if (const int te = trace_install()) return te;
 #endif
@@ -288,10 +292,7 @@ static inline int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t
 template <typename... KArgs, typename... Args>
 static inline int launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_x, Args... args) {
     if (cluster_x < 1 || grid.x % cluster_x) return static_cast<int>(cudaErrorInvalidValue);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return static_cast<int>(e);
-    }
+    if (const cudaError_t e = opt_in_smem(kernel, smem); e != cudaSuccess) return static_cast<int>(e);
 #ifdef NEXRT_TRACE
     if (const int te = trace_install()) return te;
 #endif

@@ -1,5 +1,6 @@
-"""Shared-memory layout of the CUDA-core row kernels: what lies behind the partial sums starts on a 16-byte boundary, whatever the
-numbers of rows, CTAs and threads.  The layout function is compiled for the host."""
+"""Shared memory of the row kernels.  Layout of the CUDA-core forms: what lies behind the partial sums starts on a 16-byte boundary,
+whatever the numbers of rows, CTAs and threads (the layout function is compiled for the host).  Size: launches whose dynamic
+memory alone stays within the default limit of 48 KB and whose static memory takes them over it."""
 
 import shutil
 import subprocess
@@ -119,3 +120,31 @@ def test_router_and_gate_up(H):
     assert picked[-1] == E and sorted(picked[:-1]) == sorted(logits[0, :E].topk(topk).indices.tolist())
     for s, e in enumerate(picked):
         _close(gu[s : s + 1], xn, w[e * R : (e + 1) * R])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,hd,heads,n_cta", [(4096, 256, 4, 148),      # tensor-core form: 48 KB of dynamic memory to the byte
+                                              (2304, 128, 2, 27)])      # CUDA-core form: 32 bytes below 48 KB
+def test_attn_front_of_two_rows_at_the_default_limit(H, hd, heads, n_cta):
+    import torch
+    from nexrt_b200.ops.lib import check, load, ptr
+    from nexrt_b200.quant import dequantize_blockwise, quantize_blockwise
+    from nexrt_b200.runtime.control import CTL_WORDS
+
+    M, kvh = 2, 1 if heads == 4 else 2
+    R = (2 * heads + 2 * kvh) * hd
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(M, H, device="cuda", generator=g).to(torch.bfloat16)
+    ln = 1 + 0.1 * torch.randn(H, device="cuda", generator=g)
+    wq, ws = quantize_blockwise(torch.randn(R, H, device="cuda", generator=g) * 0.03)
+    z = lambda *s: torch.zeros(*s, device="cuda")
+    q, gate, k, v, ctl = z(M, heads, hd), z(M, heads, hd), z(M, kvh, hd), z(kvh, 4, hd).to(torch.bfloat16), torch.zeros(CTL_WORDS, dtype=torch.int32, device="cuda")
+    check(load().nexrt_attn_front(ptr(x), ptr(ln), ptr(wq), ptr(ws), ptr(ctl), ptr(q), ptr(gate), ptr(k), ptr(v), H, hd, heads, heads, kvh, M, 4, 1e-6, n_cta,
+                                  torch.cuda.current_stream().cuda_stream), "attn_front")
+    torch.cuda.synchronize()
+    xd = x.double()
+    xn, w = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * ln.double(), dequantize_blockwise(wq, ws).double()
+    pre = (xn @ w.T)[:, : (2 * heads + kvh) * hd].view(M, 2 * heads + kvh, hd)
+    got = torch.cat([torch.stack([q, gate], 2).view(M, 2 * heads, hd), k], 1).double()
+    # three e4m3 terms leave 2^-12 of an input value (2^-13 at least), random over the H products
+    assert (got - pre).abs().max() <= 4 * 2.0**-12 * xn.abs().max() * H**0.5 * 0.03
