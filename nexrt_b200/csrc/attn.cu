@@ -617,8 +617,6 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(AttnDecodeArgs a) {
 // Replaces wgmma_fd4_mega's software grid barrier + combine (nex_n2_5_pro/kernels/full_attn/
 // nex_n2_5_pro_attn_fd4_wgmma_ctypes.cu:98-118,389-401) with hardware cluster barriers; nothing here spins.
 namespace cg = cooperative_groups;
-// Keys from which the streaming form works instead of the cluster kernel (see stream_min_keys).
-constexpr int kStreamFrom = 2048, kStreamFromTwoHeads = 5120;
 constexpr int kClusterCtas = 8;       // portable cluster size
 constexpr int kClusterCtasWide = 16;  // the largest (non-portable) size: twice the warps, so one 16-key tile per warp up to 2048 keys
 
@@ -932,10 +930,9 @@ __global__ void __launch_bounds__(256) attn_decode_cluster_kernel(AttnDecodeArgs
 }
 
 // ---- streaming form (attn_stream.cuh) and its merge ----------------------------------------------------------------------
-// Both are launched behind the cluster kernel where the cache can hold more than `min_keys` keys, and the committed length
-// decides on the device which of them works: the cluster kernel up to min_keys, these two above (a launch that leaves at once
-// costs the step 0.6 us).  All of them wait for their predecessor before they leave, so the chain of dependent launches holds
-// whichever works.
+// Most calls take this form or the cluster kernel alone; which, their shape and the cache's length decide (attn_form).  Where both are
+// launched the committed length decides on the device which of them works: the cluster kernel up to min_keys, these two above.  All of
+// them wait for their predecessor before they leave, so the chain of dependent launches holds whichever works.
 //
 // One B200, one rank's heads (4 over one kv head): one row at 200K keys 60.9 us in the cluster kernel -> 41 + 4 us (205 MB,
 // 5.0 TB/s); eight rows at 32K keys, four passes over K and V, 61.7 -> 23.5 + 4.1 us.  Code that runs once is kept rolled where
@@ -1466,21 +1463,41 @@ static int launch_cluster_form(const AttnDecodeArgs& a, int hd, int kvh, int n_s
     return cudaErrorInvalidValue;
 }
 
-// Context length from which the streaming form works instead of the cluster kernel (INT_MAX: never).  It exists for head dim 256
-// and plain causal windows; context-parallel groups, sliding windows, non-causal and ungated blocks stay on the cluster kernel.
-// The lines, us a layer, cluster kernel / streaming form (B200):
-//   one kv head, up to seven passes of eight rows: up to 2048 keys the cluster kernel has one tile per warp.  One row of four
-//     heads 20.2 / 21.7 at 1100 keys, 27.0 / 22.3 at 4200; eight rows 30.3 / 38.2 and 36.8 / 36.8 (31.5 with the shorter prologue).
-//   two kv heads, one row of 16 heads each: 51.4 / 54 at 4200, 57.4 / 55.3 at 8400.
-//   from eight passes up the cluster kernel's clusters no longer fit the device together: four rows of 2 x 16 heads 101 / 72 at 64
-//     keys, 174 / 95 at 16800; eight rows 184 / 84 and 300 / 126.
-static int stream_min_keys(const AttnDecodeArgs& a, int hd, int cp_size, int window) {
-    if (hd != kStreamHd || cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate || a.rotary > hd) return INT_MAX;
+// Which form a call takes.  The streaming form exists for head dim 256 and plain causal windows; context-parallel groups, sliding
+// windows, non-causal and ungated blocks stay on the cluster kernel.  The host sees the shape and the cache's length, not the context's;
+// launching both forms and deciding on the device costs 2 to 3.5 us (the streaming kernel fills an SM's shared memory, so that nothing
+// overlaps with it).  One B200, attention layer with its weights from memory, us, cluster kernel / streaming form / both launched:
+//   one kv head, heads x rows    48 keys              1900                 4200                 17000
+//     4 x 1                      17.8 / 18.1 / 21.1   19.3 / 19.0 / 22.4   26.3 / 19.8 / 23.0   28.6 / 21.7 / 25.1
+//     8 x 1                      22.4 / 23.2 / 26.3   23.9 / 24.0 / 27.5   31.1 / 24.0 / 26.4   33.4 / 27.6 / 30.2
+//     4 x 4                      25.1 / 26.3 / 27.4   26.8 / 26.9 / 28.9   34.4 / 27.2 / 29.3   41.3 / 30.8 / 34.0
+//     4 x 8                      28.7 / 28.8 / 31.9   30.7 / 29.0 / 33.6   36.6 / 29.5 / 32.4   56.0 / 35.1 / 37.8
+//     16 x 3                     41.9 / 42.6 / 45.2   43.7 / 43.3 / 47.1   49.9 / 44.9 / 47.2   68.0 / 53.3 / 56.1
+//     16 x 1                     31.2 / 35.0 / 33.6   33.0 / 36.0 / 35.4   40.2 / 35.9 / 37.0   47.0 / 38.8 / 41.7
+//   two kv heads, 32 x 1         41.8 / 52.6 / 45.8   43.9 / 51.6 / 47.5   50.1 / 53.5 / 53.3   69.0 / 60.5 / 62.1
+// * Up to 2048 keys the cluster kernel has one 16-key tile per warp: it takes caches of up to that size.
+// * Longer caches take the streaming form at whatever length the context is: it loses at most 1.2 us of a short context.
+// * Except one row of more than eight heads: the cluster kernel's launch overlaps with the wide front and lets the wide out-projection
+//   load its weights early, the streaming kernel's does neither.  There the lines, below which the cluster kernel works alone, lie at
+//   3072 keys (its second cluster) and 11264 keys (57.1 / 57.0 at 9000, 60.7 / 58.2 at 12000); longer caches meet both sides of them, and
+//   both forms are launched.
+// * From eight passes of eight rows on the cluster kernel's clusters no longer fit the device together, and the streaming form takes
+//   every cache.  Four rows of 2 x 16 heads 138 / 70 at 48 keys, 209 / 92 at 17000; eight rows of 8 heads over one kv head 74 / 35 and 122 / 47.
+constexpr int kClusterKeys = 2048, kClusterKeysWideRow = 3072, kClusterKeysTwoHeads = 11264;
+struct AttnForm {
+    bool cluster, stream;
+    int line;                 // both: keys up to which the cluster kernel works
+};
+static AttnForm attn_form(const AttnDecodeArgs& a, int hd, int cp_size, int window) {
+    const AttnForm cluster{true, false, INT_MAX}, stream{false, true, 0};
+    if (hd != kStreamHd || cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate || a.rotary > hd) return cluster;
     const int rows = a.M * (a.nq / a.kvh);
     const size_t smem = rows <= 8 ? attn_stream_smem<1, 1>(a.M, a.rotary) : (rows <= 16 ? attn_stream_smem<2, 1>(a.M, a.rotary) : attn_stream_smem<2, 2>(a.M, a.rotary));
-    if (smem > 227 * 1024) return INT_MAX;
-    const int passes = a.kvh * ((rows + kRowsPerPassMma - 1) / kRowsPerPassMma);
-    return passes >= 8 ? 0 : (a.kvh == 1 ? kStreamFrom : kStreamFromTwoHeads);
+    if (smem > 227 * 1024) return cluster;
+    if (a.kvh * ((rows + kRowsPerPassMma - 1) / kRowsPerPassMma) >= 8) return stream;
+    if (a.M > 1 || a.nq <= 8) return a.cache_len > kClusterKeys ? stream : cluster;
+    const int line = a.kvh == 1 ? kClusterKeysWideRow : kClusterKeysTwoHeads;
+    return a.cache_len > line ? AttnForm{true, true, line} : cluster;
 }
 
 template <int NTR, int WR>
@@ -1519,10 +1536,10 @@ extern "C" int nexrt_attn_decode(const void* q_raw, const void* gate, const void
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool mma = (gemv_mode() & 32) != 0;
     if (mma && (gemv_mode() & 64) && n_splits >= kClusterCtas) {
-        const int stream_from = stream_min_keys(a, hd, cp_size, window);
-        if (stream_from > 0)
-            if (const int e = launch_cluster_form(a, hd, kvh, n_splits, stream_from, st)) return e;
-        return a.cache_len > stream_from ? launch_stream_form(a, stream_from, st) : 0;
+        const AttnForm form = attn_form(a, hd, cp_size, window);
+        if (form.cluster)
+            if (const int e = launch_cluster_form(a, hd, kvh, n_splits, form.line, st)) return e;
+        return form.stream ? launch_stream_form(a, form.line, st) : 0;
     }
     a.flags &= ~8;   // only the cluster kernel reads the control block before its dependency wait
     const int passes = (M * (nq / kvh) + kRowsPerPassMma - 1) / kRowsPerPassMma;     // tensor-core path: eight query rows per CTA
