@@ -94,10 +94,14 @@ class FullAttn:
             wide.oproj_allreduce(c, c.attn_out, c.gate, None, self.w["out_w"], self.w["out_s"], spec.attn_local, M, 2 if merge_here else 0, cfg.head_dim,
                                  c.cp_channel.ref if merge_here else None, cp_site)
             return
+        # One row of 4096 inputs: a staging kernel in front of the projection gains behind the streaming form's merge kernel (37.4 us a layer
+        # at 1100 keys with it, 39.9 without: B200), but not behind the cluster kernel (32.4, 31.5)
+        cluster = use_cp or self.cache_len <= lib.nexrt_attn_cluster_keys(cfg.head_dim, nq, spec.kv_heads, M, cfg.rotary_dim)
+        planes = None if M == 1 and spec.attn_local <= 4096 and cluster else ptr(c.oproj_planes)
         check(
             lib.nexrt_oproj_rows_allreduce(
                 ptr(c.attn_out), ptr(c.gate), None, ptr(self.w["out_w"]), ptr(self.w["out_s"]), ptr(c.x),
-                ptr(c.oproj_planes), ptr(c.oproj_descale), cfg.hidden, spec.attn_local, M,
+                planes, ptr(c.oproj_descale), cfg.hidden, spec.attn_local, M,
                 2 if merge_here else 0, cfg.rms_eps, cfg.head_dim, c.ar_channel.ref, c.next_site(), c.cp_channel.ref if merge_here else None, cp_site,
                 n_cta, st,
             ),

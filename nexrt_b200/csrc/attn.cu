@@ -1484,20 +1484,29 @@ static int launch_cluster_form(const AttnDecodeArgs& a, int hd, int kvh, int n_s
 // * From eight passes of eight rows on the cluster kernel's clusters no longer fit the device together, and the streaming form takes
 //   every cache.  Four rows of 2 x 16 heads 138 / 70 at 48 keys, 209 / 92 at 17000; eight rows of 8 heads over one kv head 74 / 35 and 122 / 47.
 constexpr int kClusterKeys = 2048, kClusterKeysWideRow = 3072, kClusterKeysTwoHeads = 11264;
+// Keys up to which the cluster kernel is the form to take for these shapes (0: none, INT_MAX: there is no other form).
+static int cluster_keys(int hd, int nq, int kvh, int M, int rotary) {
+    if (hd != kStreamHd || rotary > hd) return INT_MAX;
+    const int rows = M * (nq / kvh);
+    const size_t smem = rows <= 8 ? attn_stream_smem<1, 1>(M, rotary) : (rows <= 16 ? attn_stream_smem<2, 1>(M, rotary) : attn_stream_smem<2, 2>(M, rotary));
+    if (smem > 227 * 1024) return INT_MAX;
+    if (kvh * ((rows + kRowsPerPassMma - 1) / kRowsPerPassMma) >= 8) return 0;
+    return M > 1 || nq <= 8 ? kClusterKeys : (kvh == 1 ? kClusterKeysWideRow : kClusterKeysTwoHeads);
+}
 struct AttnForm {
     bool cluster, stream;
     int line;                 // both: keys up to which the cluster kernel works
 };
 static AttnForm attn_form(const AttnDecodeArgs& a, int hd, int cp_size, int window) {
     const AttnForm cluster{true, false, INT_MAX}, stream{false, true, 0};
-    if (hd != kStreamHd || cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate || a.rotary > hd) return cluster;
-    const int rows = a.M * (a.nq / a.kvh);
-    const size_t smem = rows <= 8 ? attn_stream_smem<1, 1>(a.M, a.rotary) : (rows <= 16 ? attn_stream_smem<2, 1>(a.M, a.rotary) : attn_stream_smem<2, 2>(a.M, a.rotary));
-    if (smem > 227 * 1024) return cluster;
-    if (a.kvh * ((rows + kRowsPerPassMma - 1) / kRowsPerPassMma) >= 8) return stream;
-    if (a.M > 1 || a.nq <= 8) return a.cache_len > kClusterKeys ? stream : cluster;
-    const int line = a.kvh == 1 ? kClusterKeysWideRow : kClusterKeysTwoHeads;
-    return a.cache_len > line ? AttnForm{true, true, line} : cluster;
+    if (cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate) return cluster;
+    const int line = cluster_keys(hd, a.nq, a.kvh, a.M, a.rotary);
+    if (a.cache_len <= line) return cluster;
+    return line <= kClusterKeys ? stream : AttnForm{true, true, line};
+}
+extern "C" int nexrt_attn_cluster_keys(int hd, int nq, int kvh, int M, int rotary) {
+    const bool streams = (gemv_mode() & 32) && (gemv_mode() & 64) && kvh > 0 && nq >= kvh && M > 0;
+    return streams ? cluster_keys(hd, nq, kvh, M, rotary) : INT_MAX;
 }
 
 template <int NTR, int WR>

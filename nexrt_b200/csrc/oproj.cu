@@ -423,9 +423,10 @@ extern "C" int nexrt_oproj_allreduce(const void* in, const void* z, const void* 
 }
 
 // The same with scratch for the input's terms (planes: e4m3 [3 M][K], descale: fp32 [M]): made once by a kernel of their own
-// instead of by every CTA.  The line: several rows always gain (see above); one row gains where K is wide - an unsharded
-// 8192 takes 4.0 + 8.1 us against 14.6, 4096 a layer of 29.1 us against 30.8, 2048 no difference, and at 1024 the second
-// node costs more than the eight blocks that every CTA computes.
+// instead of by every CTA.  The line: several rows always gain (see above); one row gains where K is wide (one B200, a layer with its weights
+// from memory, staged / not: K = 8192 41.8 / 44.0 us of attention and 42.7 / 46.5 of gated delta net, K = 4096 28.8 / 29.0 of gated delta
+// net; of attention it depends on the kernel in front, see FullAttn).  At 2048 there is no difference, and at 1024 the second node costs
+// more than the eight blocks that every CTA computes.
 extern "C" int nexrt_oproj_rows_allreduce(const void* in, const void* z, const void* gnorm_w, const void* w, const void* s, void* x, void* planes, void* descale,
                                           int H, int K, int M, int mode, float eps, int hd, const NexrtLLChannel* ch, unsigned int site,
                                           const NexrtLLChannel* cp, unsigned int cp_site, int n_cta, void* stream) {

@@ -30,6 +30,12 @@ def test_lines_between_the_forms(M, nq, kvh, keys, cache):
     _check_decode(M, nq, kvh, keys - M, cache)
 
 
+@pytest.mark.parametrize("hd,nq,kvh,M,keys", [(256, 4, 1, 1, 2048), (256, 8, 1, 1, 2048), (256, 4, 1, 8, 2048), (256, 16, 1, 1, 3072), (256, 16, 1, 3, 2048), (256, 32, 2, 1, 11264),
+                                              (256, 16, 1, 4, 0), (256, 32, 2, 2, 0), (256, 8, 1, 8, 0), (128, 4, 1, 1, 2**31 - 1)])
+def test_keys_of_the_cluster_kernel(hd, nq, kvh, M, keys):
+    assert load().nexrt_attn_cluster_keys(hd, nq, kvh, M, ROT) == keys
+
+
 def _check_decode(M, nq, kvh, C0, cache):
     g = torch.Generator(device=DEV).manual_seed(M * 1000 + nq + C0)
     n_splits, G, end = 148 // kvh, nq // kvh, min(C0 + M, cache)
