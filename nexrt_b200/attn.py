@@ -21,7 +21,7 @@ import torch
 
 from .ops import wide
 from .ops.lib import NOT_SUPPORTED, check, ptr
-from .runtime.context import StepContext
+from .runtime.context import NEAR, StepContext
 
 
 class FullAttn:
@@ -76,7 +76,7 @@ class FullAttn:
         # bit 8: the kernel may read the committed length before its dependency wait - true for the engine's own control
         # block inside a step (its only writer is the head at the end of the step, and the step's first kernel holds its
         # dependents back until everything before the step is complete), not for a draft layer's private block
-        flags = 8 if (ctl is c.ctl and c.early_ctl) else 0
+        flags = (8 if (ctl is c.ctl and c.early_ctl) else 0) | c.attn_side
         check(
             lib.nexrt_attn_decode(
                 ptr(c.q_raw), ptr(c.gate), ptr(c.k_raw), ptr(self.w["qn"]), ptr(self.w["kn"]), ptr(c.inv_freq), ptr(c.rope_table(self.cache_len)), ptr(ctl), ptr(self.k_cache),
@@ -96,7 +96,7 @@ class FullAttn:
             return
         # One row of 4096 inputs: a staging kernel in front of the projection gains behind the streaming form's merge kernel (37.4 us a layer
         # at 1100 keys with it, 39.9 without: B200), but not behind the cluster kernel (32.4, 31.5)
-        cluster = use_cp or self.cache_len <= lib.nexrt_attn_cluster_keys(cfg.head_dim, nq, spec.kv_heads, M, cfg.rotary_dim)
+        cluster = use_cp or c.attn_side == NEAR or self.cache_len <= lib.nexrt_attn_cluster_keys(cfg.head_dim, nq, spec.kv_heads, M, cfg.rotary_dim)
         planes = None if M == 1 and spec.attn_local <= 4096 and cluster else ptr(c.oproj_planes)
         check(
             lib.nexrt_oproj_rows_allreduce(

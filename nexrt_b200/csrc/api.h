@@ -63,6 +63,7 @@ int nexrt_attn_front(const void* x, const void* in_ln, const void* w, const void
                      void* v_cache, int H, int hd, int nq, int ngate, int kvh, int M, int cache_len, float eps, int n_cta, void* stream);
 size_t nexrt_attn_decode_smem(int hd, int nq, int kvh, int M);
 int nexrt_attn_cluster_keys(int hd, int nq, int kvh, int M, int rotary);   /* keys up to which the cluster kernel is the form to take (INT_MAX: the only one) */
+int nexrt_attn_both_forms(int hd, int nq, int kvh, int M, int rotary, int cache_len);   /* 1: a call with these launches both forms unless flags 16 / 32 name the side */
 int nexrt_attn_decode(const void* q_raw, const void* gate, const void* k_raw, const void* qn, const void* kn, const void* inv_freq,
                       const void* rope_table, const void* ctl, void* k_cache, const void* v_cache, void* ws_acc, void* ws_ml, void* ticket, void* out, int hd, int nq,
                       int ngate, int kvh, int M, int cache_len, int rotary, int n_splits, float eps, int flags, int window, int ldq, int ldk,

@@ -226,7 +226,8 @@ struct AttnDecodeArgs {
     float eps;
     // context parallel
     int ldq, ldk;             // row strides of q_raw / k_raw in floats (0: packed)
-    int flags;                // 1: rows of the step see each other (non-causal block); 2: no output gate; 4: the new k rows are in the cache already; 8: control block readable before the dependency wait
+    int flags;                // 1: rows of the step see each other (non-causal block); 2: no output gate; 4: the new k rows are in the cache already; 8: control block readable before the dependency wait;
+                              // 16 / 32: the context is within / beyond nexrt_attn_cluster_keys (see attn_form)
     int window;               // > 0: sliding window, only the last `window` positions are attended
     int cp_size, cp_rank;     // window of the prefix this rank attends
     LLChannel ch;             // partial exchange inside the cp group (world == cp_size)
@@ -1480,7 +1481,8 @@ static int launch_cluster_form(const AttnDecodeArgs& a, int hd, int kvh, int n_s
 // * Except one row of more than eight heads: the cluster kernel's launch overlaps with the wide front and lets the wide out-projection
 //   load its weights early, the streaming kernel's does neither.  There the lines, below which the cluster kernel works alone, lie at
 //   3072 keys (its second cluster) and 11264 keys (57.1 / 57.0 at 9000, 60.7 / 58.2 at 12000); longer caches meet both sides of them, and
-//   both forms are launched.
+//   both forms are launched - unless the caller knows the side (flags 16: the context is within the line, 32: beyond it).
+//   That is a choice of speed only: both forms are right at every length.
 // * From eight passes of eight rows on the cluster kernel's clusters no longer fit the device together, and the streaming form takes
 //   every cache.  Four rows of 2 x 16 heads 138 / 70 at 48 keys, 209 / 92 at 17000; eight rows of 8 heads over one kv head 74 / 35 and 122 / 47.
 constexpr int kClusterKeys = 2048, kClusterKeysWideRow = 3072, kClusterKeysTwoHeads = 11264;
@@ -1499,14 +1501,19 @@ struct AttnForm {
 };
 static AttnForm attn_form(const AttnDecodeArgs& a, int hd, int cp_size, int window) {
     const AttnForm cluster{true, false, INT_MAX}, stream{false, true, 0};
-    if (cp_size > 1 || window > 0 || (a.flags & ~8) || a.ldq || a.ldk || a.nq != a.ngate) return cluster;
+    if (cp_size > 1 || window > 0 || (a.flags & ~(8 | 16 | 32)) || a.ldq || a.ldk || a.nq != a.ngate) return cluster;
     const int line = cluster_keys(hd, a.nq, a.kvh, a.M, a.rotary);
     if (a.cache_len <= line) return cluster;
-    return line <= kClusterKeys ? stream : AttnForm{true, true, line};
+    if (line <= kClusterKeys) return stream;
+    return (a.flags & 16) ? cluster : ((a.flags & 32) ? stream : AttnForm{true, true, line});
 }
 extern "C" int nexrt_attn_cluster_keys(int hd, int nq, int kvh, int M, int rotary) {
     const bool streams = (gemv_mode() & 32) && (gemv_mode() & 64) && kvh > 0 && nq >= kvh && M > 0;
     return streams ? cluster_keys(hd, nq, kvh, M, rotary) : INT_MAX;
+}
+extern "C" int nexrt_attn_both_forms(int hd, int nq, int kvh, int M, int rotary, int cache_len) {
+    const int line = nexrt_attn_cluster_keys(hd, nq, kvh, M, rotary);
+    return line > kClusterKeys && cache_len > line;
 }
 
 template <int NTR, int WR>

@@ -26,7 +26,7 @@ from .gdn import Gdn
 from .head import MODE_COMMIT, Head
 from .moe import Moe
 from .ops.lib import check, ptr
-from .runtime.context import StepContext
+from .runtime.context import FAR, NEAR, StepContext
 from .runtime.control import CTL_WORDS, Ctl, decode_ctl
 from .runtime.rounds import Stops, stop_set
 
@@ -216,13 +216,21 @@ class DecodeEngine:
         return 1 << 30
 
     # ---- graphs -------------------------------------------------------------------------------
-    def capture(self, M: int = 1, cp: bool = False, warmup: int = WARMUP_STEPS):
+    def capture(self, M: int = 1, cp: bool = False, warmup: int = WARMUP_STEPS, side: int = 0):
         """Warm up, then capture one whole step into a CUDA graph (reference
         decode_engine.py:308-324).  The control block is restored afterwards so the capture leaves
-        the sequence where it was."""
-        key = (M, bool(cp))
+        the sequence where it was.  ``side`` (``NEAR`` / ``FAR``): the graph is replayed at contexts on that side of the
+        attention line only (``StepContext.attn_side``); it is right, but slower, on the other."""
+        key = (M, bool(cp), side) if side else (M, bool(cp))
         if key in self.graphs:
             return self.graphs[key]
+        self.ctx.attn_side = side
+        try:
+            return self._capture(key, M, cp, warmup)
+        finally:
+            self.ctx.attn_side = 0
+
+    def _capture(self, key, M: int, cp: bool, warmup: int):
         saved = self._snapshot()
         side = torch.cuda.Stream(device=self.dev)
         side.wait_stream(torch.cuda.current_stream(self.dev))
@@ -241,6 +249,20 @@ class DecodeEngine:
         if self.world > 1:
             dist.barrier(group=self.group)
         return g
+
+    def _plain_graphs(self, first: int, steps: int):
+        """``(line, near, far)``: one-row graphs for ``steps`` steps from committed length ``first`` on - ``near`` while a step's keys
+        are within ``line``, ``far`` behind it.  Where an attention call would launch both of its forms and let the device choose,
+        they are two graphs (of which only those needed are captured), otherwise the same one."""
+        lib, cfg, spec = self.ctx.lib, self.cfg, self.spec
+        shape = (cfg.head_dim, spec.q_heads, spec.kv_heads, 1, cfg.rotary_dim)
+        if not any(isinstance(m, FullAttn) and lib.nexrt_attn_both_forms(*shape, m.cache_len) for m in self.mixers):
+            g = self.capture(1)
+            return 0, g, g
+        line = lib.nexrt_attn_cluster_keys(*shape)
+        near = self.capture(1, side=NEAR) if first + 1 <= line else None
+        far = self.capture(1, side=FAR) if near is None or first + steps > line else None
+        return line, near or far, far or near
 
     def _snapshot(self):
         torch.cuda.synchronize(self.dev)
@@ -285,18 +307,18 @@ class DecodeEngine:
         stops = stop_set(eos)
         if cp_threshold is None:
             cp_threshold = self.cp_threshold
-        g_noncp = g_noncp or self.capture(1, cp=False)
+        S = int(self.ctx.ctl[Ctl.COMMITTED_LEN].item())
+        budget = self._kv_budget()
+        line, near, far = (0, g_noncp, g_noncp) if g_noncp else self._plain_graphs(S, min(max_new, max(1, budget - S)))
         if self.cp and g_cp is None:
             g_cp = self.capture(1, cp=True)
         self.mirror.resync()
-        S = int(self.ctx.ctl[Ctl.COMMITTED_LEN].item())
-        budget = self._kv_budget()
         out: List[int] = []
 
         def launch(pos: int) -> int:
             if host_inputs is not None:  # per-step upload of the request's sampling words (pinned host memory)
                 self.ctx.sampling.copy_(host_inputs, non_blocking=True)
-            (g_cp if (g_cp is not None and pos >= cp_threshold) else g_noncp).replay()
+            (g_cp if (g_cp is not None and pos >= cp_threshold) else (near if pos + 1 <= line else far)).replay()
             return self.mirror.next_gen()
 
         pending = [launch(S)]
@@ -360,7 +382,7 @@ class DecodeEngine:
             n = min(chunk, len(ids) - pos)
             self.set_rows(ids[pos : pos + n])
             self.set_forced_commit(n)
-            g = self.graphs.get((n, False))
+            g = self.graphs.get((n, False)) or self.graphs.get((n, False, NEAR)) or self.graphs.get((n, False, FAR))
             if g is not None:
                 g.replay()
             else:

@@ -57,6 +57,7 @@ _PROTOTYPES = {
     "nexrt_attn_front": [vp] * 9 + [ci] * 7 + [cf, ci, vp],
     "nexrt_attn_decode_merges_cp": [ci],
     "nexrt_attn_cluster_keys": [ci] * 5,
+    "nexrt_attn_both_forms": [ci] * 6,
     "nexrt_attn_decode": [vp] * 14 + [ci] * 8 + [cf, ci, ci, ci, ci, ci, ci, CH, cu, vp],
     "nexrt_oproj_allreduce": [vp] * 6 + [ci] * 4 + [cf, ci, CH, cu, CH, cu, ci, vp],
     "nexrt_oproj_rows_allreduce": [vp] * 8 + [ci] * 4 + [cf, ci, CH, cu, CH, cu, ci, vp],

@@ -21,6 +21,9 @@ MAX_ROWS = 8
 MAX_TOPK = 28
 
 
+NEAR, FAR = 16, 32    # flags of nexrt_attn_decode
+
+
 class StepContext:
     def __init__(self, cfg: ModelConfig, spec: ShardSpec, device: torch.device, group=None, budget_ms=None, cp: bool = False,
                  comm_world=None, comm_rank=None, collective: str = "fused"):
@@ -116,6 +119,9 @@ class StepContext:
         self.site = 0
         self._rope = {}
         self.early_ctl = os.environ.get("NEXRT_EARLY_CTL", "1") != "0"
+        # What the host knows about the contexts of the attention launches that follow: NEAR - at most nexrt_attn_cluster_keys keys,
+        # FAR - more, 0 - nothing.  Only speed depends on it.
+        self.attn_side = 0
 
     def canaries_violated(self):
         """Names of the scratch buffers whose guard bands were written (``NEXRT_CANARY=1`` only; ``None`` when off)."""

@@ -52,7 +52,7 @@ def _check_decode(M, nq, kvh, C0, cache):
     ctl[Ctl.COMMITTED_LEN] = C0
     ws_acc, ws_ml = torch.full((kvh, n_splits, 8 * G, HD), float("nan"), device=DEV), torch.full((kvh, n_splits, 8 * G, 2), float("nan"), device=DEV)
     ticket, out = torch.zeros(kvh, dtype=torch.int32, device=DEV), torch.zeros(8, nq * HD, device=DEV)
-    for flags in (8, 0):
+    for flags in (8, 0, 16, 8 | 32):                            # the last two: the caller names the side of the line, rightly or not
         out.zero_()
         kcc = kc.clone()
         check(load().nexrt_attn_decode(ptr(q), ptr(gate), ptr(k), ptr(qn), ptr(kn), ptr(inv), ptr(rope), ptr(ctl), ptr(kcc), ptr(vc), ptr(ws_acc), ptr(ws_ml), ptr(ticket),
