@@ -25,7 +25,7 @@ def _close(got, want, xn, what):
     assert (got.double() - want).abs().max() <= bound, (what, (got.double() - want).abs().max(), bound)
 
 
-@pytest.mark.parametrize("H,nqk,nv,M,C0", [(256, 1, 1, 2, 0), (1024, 1, 2, 5, 14), (4096, 2, 8, 8, 979), (4096, 2, 8, 3, 1), (4096, 8, 32, 2, 40), (4096, 8, 32, 6, 29)])
+@pytest.mark.parametrize("H,nqk,nv,M,C0", [(256, 1, 1, 2, 0), (1024, 1, 2, 5, 14), (4096, 2, 8, 8, 979), (4096, 2, 8, 3, 1), (4096, 8, 32, 2, 40), (4096, 8, 32, 6, 29), (4096, 2, 8, 2, 13)])
 def test_gdn_front_rows(H, nqk, nv, M, C0):
     g = torch.Generator(device=DEV).manual_seed(H + nv + M)
     C, R, ring = (2 * nqk + nv) * 128, (2 * nqk + 2 * nv) * 128, 16
@@ -62,7 +62,7 @@ def test_gdn_front_rows(H, nqk, nv, M, C0):
     assert not qkv[M:].any() and not zz[M:].any() and not beta[M:].any()
 
 
-@pytest.mark.parametrize("H,hd,nq,ngate,kvh,M,C0", [(256, 128, 1, 1, 1, 2, 0), (4096, 256, 4, 4, 1, 8, 100), (4096, 256, 16, 4, 1, 3, 7), (4096, 256, 32, 32, 2, 7, 28)])
+@pytest.mark.parametrize("H,hd,nq,ngate,kvh,M,C0", [(256, 128, 1, 1, 1, 2, 0), (4096, 256, 4, 4, 1, 8, 100), (4096, 256, 16, 4, 1, 3, 7), (4096, 256, 32, 32, 2, 7, 28), (4096, 256, 4, 4, 1, 2, 30)])
 def test_attn_front_rows(H, hd, nq, ngate, kvh, M, C0):
     g = torch.Generator(device=DEV).manual_seed(H + nq + M)
     R, cache = (nq + ngate + 2 * kvh) * hd, C0 + 4          # the last rows of a step may lie past the end of the cache

@@ -1,5 +1,6 @@
 """Grouped experts of a prefill chunk: the plan against a host sort, the persistent GEMM against float64, with experts nobody is
-routed to, experts of more pairs than one item holds, CTAs with no, one and many tiles, and one and several K blocks."""
+routed to, experts of more pairs than one item holds, CTAs with no, one and many tiles, and one and several K blocks; the activation
+of the pairs; and the whole block from the rows to what is added to the residual."""
 
 import pytest
 import torch
@@ -61,3 +62,68 @@ def test_plan_and_group_gemm(T, S, E, R, K, terms, skew):
                 w = dequantize_blockwise(wq[e], ws[e]).double()
                 y, mag = x[sel] @ w.T, x[sel].abs() @ w.abs().T
                 assert ((got[sel].double() - y).abs() <= 1e-5 * mag).all(), (e, ((got[sel].double() - y).abs() / mag).max())   # fp32 sums of up to K exact products
+
+
+def _plan(lib, ids, S, T, n_total, terms, st):
+    i32 = lambda *s: torch.full(s, -1, dtype=torch.int32, device=DEV)
+    items, n_items, pair_row, out_row = i32(T * S, 4), i32(1), i32(T * S), i32(T * S)
+    check(lib.nexrt_moe_plan(ptr(ids), ptr(items), ptr(n_items), ptr(pair_row), ptr(out_row), S, T, n_total, terms, st), "plan")
+    return items, n_items, pair_row, out_row
+
+
+# relative error of a value written as 1, 2 or 3 e4m3 terms with a scale per 128 of them: 2^-4, 2^-8, 2^-12 of the largest
+TOL = {1: 0.04, 2: 3e-3, 3: 2e-4}
+
+
+@pytest.mark.parametrize("T,S,E,I,terms", [(16, 2, 4, 128, 1), (17, 5, 16, 128, 3), (24, 3, 40, 384, 2), (128, 11, 512, 128, 3), (64, 11, 512, 1024, 3)])
+def test_pair_act(T, S, E, I, terms):
+    g = torch.Generator().manual_seed(T + I)
+    lib, st, pairs = load(), torch.cuda.current_stream().cuda_stream, T * S
+    *_, pair_row, out_row = _plan(lib, _ids(g, T, S, E, False).to(DEV), S, T, E + 1, terms, st)
+    gd = torch.Generator(device=DEV).manual_seed(T)
+    gu, wts = torch.randn(pairs, 2 * I, device=DEV, generator=gd), torch.rand(T, S, device=DEV, generator=gd) + 0.01
+    gu[:, : I // 2] *= 1e-3                                      # blocks of other magnitudes
+    hq, hs = torch.zeros(terms * pairs, I, dtype=torch.float8_e4m3fn, device=DEV), torch.zeros(pairs, I // 128, device=DEV)
+    check(lib.nexrt_moe_pair_act(ptr(gu), ptr(out_row), ptr(wts), ptr(hq), ptr(hs), I, S, T, terms, st), "pair_act")
+    torch.cuda.synchronize()
+    slot, row = out_row.long() // T, out_row.long() % T
+    assert torch.equal(row, pair_row.long())
+    want = torch.nn.functional.silu(gu[:, :I].double()) * gu[:, I:].double() * wts[row, slot].double()[:, None]
+    got = sum(hq.double().view(pairs, terms, I)[:, p] * 16.0**-p for p in range(terms)) * hs.double().repeat_interleave(128, 1)
+    err = (got - want).view(-1, 128).norm(dim=1) / want.view(-1, 128).norm(dim=1)      # every pair and block by itself
+    assert err.max() <= TOL[terms], err.max()
+
+
+@pytest.mark.parametrize("T,S,E,H,I,terms", [(16, 3, 8, 256, 128, 1), (64, 11, 512, 512, 128, 3), (128, 11, 64, 256, 256, 2), (64, 5, 12, 1024, 384, 3)])
+def test_rows_to_residual(T, S, E, H, I, terms):
+    from nexrt_b200.ops.tc_gemm import act_quant
+
+    g = torch.Generator().manual_seed(H + I)
+    gd = torch.Generator(device=DEV).manual_seed(H + I)
+    lib, st, pairs, n_total = load(), torch.cuda.current_stream().cuda_stream, T * S, E + 1
+    ids = _ids(g, T, S, E, False).to(DEV)
+    x, wts = torch.randn(T, H, device=DEV, generator=gd), torch.rand(T, S, device=DEV, generator=gd)
+    w13, s13 = quantize_blockwise(torch.randn(n_total, 2 * I, H, device=DEV, generator=gd) * 0.05)
+    w2, s2 = quantize_blockwise(torch.randn(n_total, H, I, device=DEV, generator=gd) * 0.05)
+    xq, sx = act_quant(x, terms=terms)
+    items, n_items, pair_row, out_row = _plan(lib, ids, S, T, n_total, terms, st)
+    f8, f32 = lambda *s: torch.zeros(*s, dtype=torch.float8_e4m3fn, device=DEV), lambda *s: torch.full(s, float("nan"), device=DEV)
+    xp, sp, gu, hq, hs, y, out = f8(terms * pairs, H), f32(pairs, H // 128), f32(pairs, 2 * I), f8(terms * pairs, I), f32(pairs, I // 128), f32(S * T, H), f32(T, H)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    check(lib.nexrt_moe_gather(ptr(xq), ptr(sx), ptr(pair_row), ptr(xp), ptr(sp), pairs, T, H, terms, st), "gather")
+    check(lib.nexrt_moe_group_gemm(ptr(w13), ptr(s13), ptr(xp), ptr(sp), ptr(gu), ptr(items), ptr(n_items), None, pairs, n_total, 2 * I, H, terms, ptr(status), st), "up")
+    check(lib.nexrt_moe_pair_act(ptr(gu), ptr(out_row), ptr(wts), ptr(hq), ptr(hs), I, S, T, terms, st), "pair_act")
+    check(lib.nexrt_moe_group_gemm(ptr(w2), ptr(s2), ptr(hq), ptr(hs), ptr(y), ptr(items), ptr(n_items), ptr(out_row), pairs, n_total, H, I, terms, ptr(status), st), "down")
+    check(lib.nexrt_planes_residual(None, ptr(y), ptr(out), T * H, S, st), "planes_sum")
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    want = torch.zeros(T, H, dtype=torch.float64, device=DEV)
+    for e in range(n_total):
+        row, slot = (ids == e).nonzero(as_tuple=True)
+        if len(row):
+            u = x[row].double() @ dequantize_blockwise(w13[e], s13[e]).double().T
+            h = torch.nn.functional.silu(u[:, :I]) * u[:, I:] * wts[row, slot].double()[:, None]
+            want.index_add_(0, row, h @ dequantize_blockwise(w2[e], s2[e]).double().T)
+    # the rounding of the rows reaches gate and up, that of h comes on top
+    err = (out.double() - want).norm(dim=1) / want.norm(dim=1)
+    assert err.max() <= 4 * TOL[terms], err.max()

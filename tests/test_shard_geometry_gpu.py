@@ -63,7 +63,7 @@ def test_one_row_steps_at_deployment_shapes(setup):
     assert ctl["committed_len"] == len(prompt) and ctl["status"] == 0
 
 
-@pytest.mark.parametrize("rows", [4, 8])
+@pytest.mark.parametrize("rows", [2, 4, 8])     # 2: the ragged end of a prompt
 def test_verify_rows_at_deployment_shapes(setup, rows):
     """The speculative verifiers' row counts (tcgen05 experts, wide fronts, multi-row attention)."""
     cfg, ref, eng = setup
@@ -97,3 +97,14 @@ def test_graph_replay_at_deployment_shapes(setup):
     eng.load_prefill(state)
     assert eng.read_ctl()["pending"] == first
     assert eng.generate(max_new=5) == eager
+
+
+def test_prompt_that_ends_on_two_rows(setup):
+    """A prompt of 8 n + 2 tokens: the last prefill step has two rows.  Same logits as the oracle's last token."""
+    cfg, ref, eng = setup
+    prompt, margin = robust_prompt(ref, cfg.vocab, 10, seeds=range(30, 38))
+    ref.reset()
+    want = [ref.step(t) for t in prompt][-1]
+    eng.prefill(prompt, chunk=8)
+    _check(gather_logits(eng, 2)[1], want)
+    assert eng.read_ctl()["committed_len"] == len(prompt)
