@@ -1,9 +1,11 @@
 """Gated full-attention layer block (non-CP and context-parallel arms).
 
 Counterpart of the reference's ``FullAttn`` (``nex_n2_5_pro/attn.py:261-512``) and ``FullAttnCP``
-(``nex_n2_5_pro/attn_cp.py:76-367``).  Three launches per layer: projection front (v appended to
-the cache), split-KV decode (q/k norm + RoPE in its prologue, combine by the last CTA), and the
-out-projection fused with the all-reduce and the residual.  In the context-parallel arm the
+(``nex_n2_5_pro/attn_cp.py:76-367``).  Projection front (v appended to the cache), split-KV decode
+(q/k norm + RoPE in its prologue), and the out-projection fused with the all-reduce and the
+residual: three launches for one row and a short cache.  A long cache adds the kernel that merges
+the splits (a short one's cluster does that itself), several rows the kernels that make the terms of
+a projection's input once for all CTAs.  In the context-parallel arm the
 front also projects the q heads of the other ranks that share this rank's kv head (the
 reference's duplicate-Q weights, ``attn.py:220-257``), the decode kernel attends only this
 rank's window of the prefix and sends per-head partials to their owners, and the LSE merge runs

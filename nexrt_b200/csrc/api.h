@@ -89,8 +89,7 @@ int nexrt_moe_l1(const void* x, const void* post_ln, const void* w13, const void
 /* routed pair of the one-row step: the router stops at K-split partial logits [split][M][rows_pad]; the gate/up kernel adds
  * them, selects the experts in every CTA and leaves ids / weights / logits for the down projection */
 int nexrt_moe_router_partial(const void* x, const void* post_ln, const void* w, void* partial, int rows_pad, int H, int E, int topk, int M,
-                             float eps, void* planes, void* stream);
-int nexrt_moe_router_partial_split(void);
+                             float eps, void* stream);
 int nexrt_moe_l1_routed(const void* x, const void* post_ln, const void* w13, const void* w13_s, const void* partial, int rows_pad, void* ids_out,
                         void* wts_out, void* logits_out, void* gu, const void* w2, const void* pf, unsigned long long pf_bytes, int H, int I,
                         int E, int topk, int M, float eps, void* stream);
@@ -163,7 +162,7 @@ int nexrt_moe_plan(const void* ids, void* items, void* n_items, void* pair_row, 
 int nexrt_moe_gather(const void* xq, const void* sx, const void* pair_row, void* xp, void* sp, int pairs, int T, int K, int terms, void* stream);
 int nexrt_moe_group_gemm(const void* w, const void* w_s, const void* xp, const void* sp, void* out, const void* items, const void* n_items, const void* out_row,
                          int pairs, int n_total, int R, int K, int terms, int* status, void* stream);
-int nexrt_moe_pair_act(const void* gu, const void* out_row, const void* wts, void* hq, void* hs, int I, int S, int T, int terms, void* stream);   /* used[e] = 1 for every routed expert id */
+int nexrt_moe_pair_act(const void* gu, const void* out_row, const void* wts, void* hq, void* hs, int I, int S, int T, int terms, void* stream);   /* h of every pair: gu [pairs][2I] -> hq [pairs * terms][I], hs [pairs][I / 128] */
 int nexrt_planes_residual(void* x, const void* y, void* sum_out, int64_t n, int ksplit, void* stream);
 int nexrt_gdn_chunk(const void* pre, const void* xn, const void* ba_w, const void* conv_w, const void* a_log, const void* dt_bias, const void* ctl,
                     void* conv_ring, void* qkv, void* z, void* beta, void* g, void* state_ring, void* out, int H, int R, int C, int nv, int nqk, int T,
@@ -179,8 +178,7 @@ int nexrt_tc_moe_l2_allreduce(const void* gu, const void* ids, const void* wts, 
                               int H, int I, int S, int M, int n_experts_total, int gu_ksplit, const NexrtLLChannel* ch, unsigned int site, int* status,
                               void* stream);
 
-// ---- wide (multi-row) projections on tcgen05 ---------------------------------------------------------------------
-   /* out: [ksplit][M][R] partial planes */
+// ---- projections of several rows ---------------------------------------------------------------------------------
 int nexrt_gdn_front_rows(const void* x, const void* in_ln, const void* front_w, const void* front_s, const void* ba_w, const void* conv_w, const void* a_log,
                          const void* dt_bias, const void* ctl, void* conv_ring, void* qkv, void* z, void* beta, void* g, void* cols, int H, int R, int C,
                          int nv, int M, int conv_ring_len, float eps, void* stream);   /* 2..8 rows; cols: f16 [2 M][H] scratch */
@@ -190,20 +188,22 @@ int nexrt_attn_front_rows(const void* x, const void* in_ln, const void* w, const
 int nexrt_tc_router_logits(const void* x, const void* gamma, const void* w, void* planes, void* partial, const void* zero_ids, int rows, int rows_pad, int K,
                            int M, int ksplit, float eps, void* planes_e4m3, int* status, void* stream);   /* partial: [ksplit][M][rows_pad] */
 int nexrt_moe_router_rows(const void* x, const void* post_ln, const void* w, void* cols, void* partial, void* planes_e4m3, int rows_pad, int H, int M, float eps,
-                          void* stream);   /* 2..8 rows; cols: bf16 [2 M][H] scratch, partial: [4][M][rows_pad] */
+                          void* stream);   /* 2..8 rows; cols: bf16 [2 M][H] scratch, partial: [split][M][rows_pad] */
+int nexrt_moe_router_rows_split(void);   /* K ranges of those partial logits */
 int nexrt_moe_router_topk(const void* partial, int ksplit, int rows_pad, void* logits, void* ids, void* wts, int E, int topk, int M, void* stream);
 
 int nexrt_lmhead_sample_from_logits(const void* logits_in, void* cand, void* ticket, const void* sampling, void* ctl, void* export_buf, int H, int V_local,
                                     int vocab_base, int M, int mode, int arg, const NexrtLLChannel* ch, unsigned int site, int n_cta, void* stream);
 
-// Wide out-projection (multi-row steps): staging + split into planes, then tcgen05 GEMM with all-reduce epilogue.
+// Out-projection in two kernels: the input's terms (also the first kernel of nexrt_oproj_rows_allreduce), and the product on tcgen05 with
+// the all-reduce in its epilogue.
 int nexrt_oproj_stage_split(const void* in, const void* z, const void* gnorm_w, void* planes, void* descale, int K, int M, int mode, float eps, int hd,
                             const NexrtLLChannel* cp, unsigned int cp_site, void* stream);
 int nexrt_tc_oproj_allreduce(const void* planes, const void* descale, const void* w, const void* w_s, void* x, const void* zero_ids, int H, int K, int M,
                              int overwrite, const NexrtLLChannel* ch, unsigned int site, int* status, void* stream);
 
 int nexrt_attn_front_tail(const void* pre, const void* ctl, void* q_raw, void* gate, void* k_raw, void* v_cache, int hd, int nq, int ngate, int kvh, int M,
-                          int cache_len, int ksplit, void* stream);   /* pre: [ksplit][M][R] partial planes of the rows GEMM */
+                          int cache_len, int ksplit, void* stream);   /* pre: [ksplit][M][R] partial planes of a chunk's GEMM */
 
 #ifdef __cplusplus
 }

@@ -1380,14 +1380,10 @@ extern "C" int nexrt_attn_front(const void* x, const void* in_ln, const void* w,
                     static_cast<float*>(k_raw), static_cast<__nv_bfloat16*>(v_cache), H, hd, nq, ngate, kvh, M, cache_len, eps};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int R = (nq + ngate + 2 * kvh) * hd;
-    if ((gemv_mode() & 1) && H % 512 == 0 && H <= 4096) {
-        const int mp = M == 1 ? 1 : (M == 2 ? 2 : 4), terms = 3;
-        const size_t smem_mma = sizeof(float) * 8 * 256 + static_cast<size_t>(mp) * terms * H + sizeof(float) * H;
-        dim3 g(R / 16), b(256);
-        if (mp == 1 && R / 16 > 2 * n_cta) return launch(attn_front_mma_kernel<1, true>, dim3(2 * n_cta), b, smem_mma, st, a);   // capped: the kernel walks the rest
-        if (mp == 1) return launch(attn_front_mma_kernel<1>, g, b, smem_mma, st, a);
-        if (mp == 2) return launch(attn_front_mma_kernel<2>, g, b, smem_mma, st, a);
-        return launch(attn_front_mma_kernel<4>, g, b, smem_mma, st, a);
+    if (M == 1 && (gemv_mode() & 1) && H % 512 == 0 && H <= 4096) {      // several rows: nexrt_attn_front_rows
+        const size_t smem_mma = sizeof(float) * 8 * 256 + static_cast<size_t>(3) * H + sizeof(float) * H;
+        if (R / 16 > 2 * n_cta) return launch(attn_front_mma_kernel<1, true>, dim3(2 * n_cta), dim3(256), smem_mma, st, a);   // capped: the kernel walks the rest
+        return launch(attn_front_mma_kernel<1>, dim3(R / 16), dim3(256), smem_mma, st, a);
     }
     const int mb = M == 1 ? 1 : 4;
     const size_t smem = sizeof(float) * (static_cast<size_t>(mb + 1) * H + gemv_part_floats((R + n_cta - 1) / n_cta, mb, gemv_geom(H / 16, gemv_threads())));

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(512, 1) gdn_front_kernel(GdnFrontArgs a) {
 
 // Tensor-core form of the front: one CTA per 16 weight rows, the 8 warps split K, FP8 weights go
 // from global memory to registers to mma.m16n8k32 against the exact e4m3 split of the normalised
-// activation.  MP token rows per pass (1, 2 or 4).  The first 2*nv CTAs also do one b/a row each.
+// activation.  One token row (MP = 1; several: gdn_front_rows_kernel).  The first 2*nv CTAs also do one b/a row each.
 #define NEXRT_EVENT(i) do { if (a.events != nullptr && blockIdx.x == 0 && threadIdx.x == 0) a.events[i] = globaltimer_ns(); } while (0)
 
 // LOOP: the grid is smaller than the number of 16-row groups and a CTA walks several of them (one-row steps on wide shards);
@@ -485,16 +485,12 @@ extern "C" int nexrt_gdn_front(const void* x, const void* in_ln, const void* fro
                    static_cast<float*>(conv_ring), static_cast<float*>(qkv), static_cast<float*>(z), static_cast<float*>(beta),
                    static_cast<float*>(g), H, R, C, nv, M, conv_ring_len, eps, ba_rows_pad, g_events};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if ((gemv_mode() & 1) && R % 16 == 0 && H % 512 == 0 && H <= 4096 && R / 16 >= 2 * nv) {
-        const int mp = M == 1 ? 1 : (M == 2 ? 2 : 4);
-        const size_t smem = sizeof(float) * (static_cast<size_t>(mp) * H + 8 * 256 + 64) + static_cast<size_t>(mp) * 3 * H + sizeof(float) * H +
-                            sizeof(__nv_bfloat16) * H + 16 * sizeof(float4);
-        dim3 g(R / 16), b(256);
-        // one row: no more CTAs than the machine holds at once (two per SM), but at least the 2 nv that carry a b/a row
-        if (mp == 1 && R / 16 > max(2 * n_cta, 2 * nv)) return launch(gdn_front_mma_kernel<1, true>, dim3(max(2 * n_cta, 2 * nv)), b, smem, st, a);
-        if (mp == 1) return launch(gdn_front_mma_kernel<1>, g, b, smem, st, a);
-        if (mp == 2) return launch(gdn_front_mma_kernel<2>, g, b, smem, st, a);
-        return launch(gdn_front_mma_kernel<4>, g, b, smem, st, a);
+    if (M == 1 && (gemv_mode() & 1) && R % 16 == 0 && H % 512 == 0 && H <= 4096 && R / 16 >= 2 * nv) {      // several rows: nexrt_gdn_front_rows
+        const size_t smem = sizeof(float) * (static_cast<size_t>(H) + 8 * 256 + 64) + static_cast<size_t>(3) * H + sizeof(float) * H + sizeof(__nv_bfloat16) * H +
+                            16 * sizeof(float4);
+        // no more CTAs than the machine holds at once (two per SM), but at least the 2 nv that carry a b/a row
+        if (R / 16 > max(2 * n_cta, 2 * nv)) return launch(gdn_front_mma_kernel<1, true>, dim3(max(2 * n_cta, 2 * nv)), dim3(256), smem, st, a);
+        return launch(gdn_front_mma_kernel<1>, dim3(R / 16), dim3(256), smem, st, a);
     }
     const int mb = M == 1 ? 1 : 4;
     const size_t smem = sizeof(float) * (static_cast<size_t>(mb + 1) * H + gemv_part_floats((R + n_cta - 1) / n_cta, mb, gemv_geom(H / 16, gemv_threads())) +

@@ -505,8 +505,8 @@ __global__ void __launch_bounds__(256, 2) moe_router_rows_kernel(const __nv_bflo
     tr.mark(3);
 }
 
-// Top-k stage of the wide router (multi-row steps): the logits arrive as K-split partial planes
-// partial[ks][m][rows_pad] from the tcgen05 rows GEMM; they are added in a fixed order into shared memory, kept
+// Top-k stage of several rows: the logits arrive as K-split partial planes partial[ks][m][rows_pad] (from the rows router of a
+// step, from the GEMMs of a prefill chunk); they are added in a fixed order into shared memory, kept
 // in a.logits for inspection, and selected exactly like the fused router does.
 __global__ void __launch_bounds__(256) moe_topk_rows_kernel(RouterArgs a, int ksplit, int rpc) {
     extern __shared__ __align__(16) float lg_s[];
@@ -746,7 +746,7 @@ extern "C" int nexrt_moe_router(const void* x, const void* post_ln, const void* 
     return launch(moe_router_kernel<4>, dim3(n_cta), dim3(gemv_threads()), smem, st, a);
 }
 
-// Partial router logits of 2..8 rows (partial: [4][M][rows_pad], for nexrt_moe_router_topk with ksplit 4) and the experts' terms
+// Partial router logits of 2..8 rows (partial: [nexrt_moe_router_rows_split()][M][rows_pad], for nexrt_moe_router_topk) and the experts' terms
 // planes_e4m3 [3 M][H]; cols: bf16 [2 M][H] scratch.  cudaErrorNotSupported, with nothing launched, for shapes outside this form.
 extern "C" int nexrt_moe_router_rows(const void* x, const void* post_ln, const void* w, void* cols, void* partial, void* planes_e4m3, int rows_pad, int H, int M,
                                      float eps, void* stream) {
@@ -789,7 +789,7 @@ extern "C" int nexrt_moe_l1(const void* x, const void* post_ln, const void* w13,
     return launch(moe_l1_kernel, dim3(n_cta), dim3(gemv_threads()), smem, static_cast<cudaStream_t>(stream), a);
 }
 
-extern "C" int nexrt_moe_router_partial_split(void) { return nexrt::kRouterPartialSplit; }
+extern "C" int nexrt_moe_router_rows_split(void) { return nexrt::kRouterRowsSplit; }
 
 // Routed pair of the one-row step: the router stops at its K-quarter partial logits (no ticket, no tail by one CTA) and
 // the gate/up kernel - every CTA alike - adds them, selects the experts on the warp-reduce unit and goes straight on to
@@ -797,14 +797,13 @@ extern "C" int nexrt_moe_router_partial_split(void) { return nexrt::kRouterParti
 // router it pulls [pf, pf + pf_bytes) towards L2 (constant weights of a later kernel), and once the ids are known the
 // selected experts' down weights (w2, may be null).
 extern "C" int nexrt_moe_router_partial(const void* x, const void* post_ln, const void* w, void* partial, int rows_pad, int H, int E, int topk, int M,
-                                        float eps, void* planes, void* stream) {
+                                        float eps, void* stream) {
     if (M < 1 || M > kMaxRows || E > 512 || topk < 1 || topk > 31 || topk > E || partial == nullptr || rows_pad < E + 1 || rows_pad % 16 ||
         H % 1024 || H > 4096)
         return cudaErrorInvalidValue;
     RouterArgs a{};
     a.x = static_cast<const __nv_bfloat16*>(x); a.post_ln = static_cast<const float*>(post_ln); a.w = static_cast<const __nv_bfloat16*>(w);
     a.H = H; a.E = E; a.topk = topk; a.M = M; a.eps = eps; a.partial = static_cast<float*>(partial); a.rows_pad = rows_pad; a.no_tail = 1;
-    a.planes = static_cast<uint8_t*>(planes);   // optional: the rows' e4m3 planes for the tcgen05 expert kernels (CTA m writes row m)
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int mp = M == 1 ? 1 : (M == 2 ? 2 : 4);
     const size_t smem_mma = sizeof(float) * (static_cast<size_t>(mp) * H + 8 * 128) + sizeof(__nv_bfloat16) * static_cast<size_t>(mp) * 2 * H;

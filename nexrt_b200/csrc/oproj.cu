@@ -291,10 +291,10 @@ __global__ void __launch_bounds__(MODE == 3 ? 512 : 256, MODE == 3 ? 1 : 2) opro
     tr.mark(3);
 }
 
-// Staging half of the wide out-projection (multi-row steps): one CTA per token row builds the projection's input
-// (mode 0 plain copy, 1 GDN gated RMSNorm with z, 2 context-parallel merge of the group's partials) and writes it as
-// three e4m3 planes [3M][K] plus a power-of-two scale per row - the B operand of the tcgen05 GEMM that follows
-// (nexrt_tc_oproj_allreduce in tc_moe.cu), which also does the all-reduce and the residual.
+// Staging kernel of an out-projection: one CTA per token row builds the projection's input (mode 0 plain copy, 1 GDN gated
+// RMSNorm with z, 2 context-parallel merge of the group's partials) and writes it as three e4m3 planes [3M][K] plus a
+// power-of-two scale per row, for the kernel behind it that does the product, the all-reduce and the residual:
+// oproj_allreduce_mma_kernel in mode 3, or where asked for the tcgen05 GEMM (nexrt_tc_oproj_allreduce in tc_moe.cu).
 __global__ void __launch_bounds__(1024) oproj_stage_split_kernel(OProjArgs a, uint8_t* planes, float* descale_out) {
     extern __shared__ __align__(16) float xs[];          // [K]
     __shared__ float red[32];

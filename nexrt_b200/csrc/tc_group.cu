@@ -318,15 +318,8 @@ __global__ void __launch_bounds__(256) moe_pair_act_kernel(const float* __restri
 
 template <int P>
 int launch_group(const CUtensorMap& mw, const CUtensorMap& mx, const GroupArgs& a, cudaStream_t st) {
-    static bool configured = false;
-    auto kern = tc_group_kernel<P>;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
-        if (e != cudaSuccess) return static_cast<int>(e);
-        configured = true;
-    }
     if (const cudaError_t e = pipe_budget_install()) return static_cast<int>(e);
-    return launch(kern, dim3(2 * sm_count()), dim3(kThreads), static_cast<size_t>(kGroupSmem), st, mw, mx, a);
+    return launch(tc_group_kernel<P>, dim3(2 * sm_count()), dim3(kThreads), static_cast<size_t>(kGroupSmem), st, mw, mx, a);
 }
 
 }  // namespace

@@ -1,8 +1,9 @@
 """Gated-delta-net (linear attention) layer block: weights, per-layer rings, launch sequence.
 
-Counterpart of the reference's ``Gdn`` (``nex_n2_5_pro/gdn.py:142-250``): three launches per
-layer, front -> recurrence -> out-projection fused with the tensor-parallel all-reduce and the
-residual add.  Differences: 1..8 token rows through the same kernels; the conv history and the
+Counterpart of the reference's ``Gdn`` (``nex_n2_5_pro/gdn.py:142-250``): front ->
+recurrence -> out-projection fused with the tensor-parallel all-reduce and the residual add: three
+launches for one row, and one more in front of each projection where several rows (or a wide row,
+out-projection) have their terms made once.  Differences: 1..8 token rows through the same kernels; the conv history and the
 recurrent state live in position-indexed rings (``conv_ring [R_c][C]``, ``state_ring
 [R_s][nv][128][128]``) for every mode; the input RMSNorm multiplier is applied in the kernel
 instead of being folded into re-quantised weights (``gdn.py:83-113``).

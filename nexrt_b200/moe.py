@@ -3,8 +3,9 @@
 Counterpart of the reference's ``Moe`` (``nex_n2_5_pro/moe.py:220-426``): 512 routed experts,
 top-10 with renormalised softmax weights, one shared expert gated by ``sigmoid(gate . x)``,
 intermediate-parallel sharding (every rank holds all experts, ``inter / tp`` columns of each).
-Three launches instead of four (router GEMV and top-k are one kernel) and the raw weight mode
-only: the post-attention RMSNorm multiplier is applied to the activation in the kernels, so
+One row takes three launches instead of four (the gate/up kernel selects the experts itself); several rows add the
+kernels that normalise the rows, select the experts and make the down projection's input once for all CTAs.  The raw
+weight mode only: the post-attention RMSNorm multiplier is applied to the activation in the kernels, so
 checkpoint tensors are used as stored (the reference's folded mode re-quantises every expert,
 ``moe.py:127-171``).
 """
@@ -62,8 +63,8 @@ class Moe:
         else:
             check(e, "moe_router_rows")
             self._planes_ready = True
-            check(lib.nexrt_moe_router_topk(ptr(c.moe_partial), 4, self.rows_pad, ptr(c.moe_logits), ptr(c.moe_ids), ptr(c.moe_wts), cfg.n_experts, cfg.top_k, M,
-                                            st), "moe_router_topk")
+            check(lib.nexrt_moe_router_topk(ptr(c.moe_partial), c.router_split, self.rows_pad, ptr(c.moe_logits), ptr(c.moe_ids), ptr(c.moe_wts), cfg.n_experts,
+                                            cfg.top_k, M, st), "moe_router_topk")
         self._experts(M)
 
     def _routed(self, M: int) -> None:
@@ -72,7 +73,7 @@ class Moe:
         c, w, lib = self.ctx, self.w, self.ctx.lib
         cfg, spec, st = c.cfg, c.spec, c.stream()
         check(lib.nexrt_moe_router_partial(ptr(c.x), ptr(w["post_ln"]), ptr(w["router_w_pad"]), ptr(c.moe_partial), self.rows_pad, cfg.hidden,
-                                           cfg.n_experts, cfg.top_k, M, cfg.rms_eps, None, st), "moe_router_partial")
+                                           cfg.n_experts, cfg.top_k, M, cfg.rms_eps, st), "moe_router_partial")
         pf, pf_bytes = self.prefetch if (self.prefetch is not None and M == 1) else (None, 0)
         check(lib.nexrt_moe_l1_routed(ptr(c.x), ptr(w["post_ln"]), ptr(w["w13"]), ptr(w["w13_s"]), ptr(c.moe_partial), self.rows_pad, ptr(c.moe_ids),
                                       ptr(c.moe_wts), ptr(c.moe_logits), ptr(c.moe_gu), ptr(w["w2"]) if self.prefetch_w2 else None, pf, pf_bytes,

@@ -63,7 +63,7 @@ _PROTOTYPES = {
     "nexrt_oproj_rows_allreduce": [vp] * 8 + [ci] * 4 + [cf, ci, CH, cu, CH, cu, ci, vp],
     "nexrt_moe_router": [vp] * 8 + [ci] * 5 + [cf, ci, vp, vp],
     "nexrt_moe_l1": [vp] * 6 + [ci] * 4 + [cf, ci, ci, vp],
-    "nexrt_moe_router_partial": [vp] * 4 + [ci] * 5 + [cf, vp, vp],
+    "nexrt_moe_router_partial": [vp] * 4 + [ci] * 5 + [cf, vp],
     "nexrt_moe_l1_routed": [vp] * 5 + [ci] + [vp] * 6 + [c_ulonglong] + [ci] * 5 + [cf, vp],
     "nexrt_set_partial_out": [vp],
     "nexrt_moe_l2_allreduce": [vp] * 6 + [ci] * 4 + [CH, cu, ci, vp],
@@ -136,8 +136,8 @@ def load(build: bool = True) -> ctypes.CDLL:
         fn.restype = ci
     lib.nexrt_attn_decode_smem.argtypes = [ci, ci, ci, ci]
     lib.nexrt_attn_decode_smem.restype = c_size_t
-    lib.nexrt_moe_router_partial_split.argtypes = []
-    lib.nexrt_moe_router_partial_split.restype = ci
+    lib.nexrt_moe_router_rows_split.argtypes = []
+    lib.nexrt_moe_router_rows_split.restype = ci
     lib.nexrt_launch_count.argtypes = []
     lib.nexrt_launch_count.restype = c_ulonglong
     _install_optional(lib)

@@ -99,7 +99,8 @@ class StepContext:
         self.moe_wts = z(MAX_ROWS, S)
         self.moe_gu = z(MAX_ROWS, S, 2 * spec.inter)
         self.moe_ticket = z(1, dtype=i32)
-        self.moe_partial = z(4, MAX_ROWS, (cfg.n_experts + 1 + 15) // 16 * 16)
+        self.router_split = self.lib.nexrt_moe_router_rows_split()                # K ranges of the rows router's partial logits
+        self.moe_partial = z(max(4, self.router_split), MAX_ROWS, (cfg.n_experts + 1 + 15) // 16 * 16)   # 4: the fused router's
         # scratch of the tcgen05 expert kernels (multi-row steps): e4m3 activation planes and per-row scales
         self.moe_planes1 = z(3 * MAX_ROWS, cfg.hidden, dtype=torch.uint8)
         self.moe_planes2 = z(3 * MAX_ROWS, S * spec.inter, dtype=torch.uint8)

@@ -68,7 +68,7 @@ def main() -> None:
             real = eng.ctx.lib
             for name in ("nexrt_gdn_front", "nexrt_gdn_core", "nexrt_attn_front", "nexrt_attn_decode", "nexrt_oproj_rows_allreduce", "nexrt_moe_router",
                          "nexrt_moe_l1", "nexrt_moe_l2_allreduce", "nexrt_lmhead_sample",
-                         "nexrt_gdn_front_rows", "nexrt_attn_front_rows", "nexrt_tc_router_logits", "nexrt_moe_router_topk", "nexrt_tc_moe_l1", "nexrt_tc_moe_l2_allreduce",
+                         "nexrt_gdn_front_rows", "nexrt_attn_front_rows", "nexrt_moe_router_rows", "nexrt_tc_router_logits", "nexrt_moe_router_topk", "nexrt_tc_moe_l1", "nexrt_tc_moe_l2_allreduce",
                          "nexrt_lmhead_sample_from_logits"):
                 eng.ctx.lib = _Without(real, name)
                 eng.graphs.clear()
