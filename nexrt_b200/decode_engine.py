@@ -358,7 +358,7 @@ class DecodeEngine:
         (``prefill_wide.WidePrefill``): whole chunks of that many tokens go through one tcgen05 GEMM per projection,
         the rest of the prompt (at least its last token) through the 8-row steps.  Its activations carry the decode
         kernels' exact three-term split unless ``self.wide_terms`` (or ``NEXRT_WIDE_TERMS``) is 2 or 1 (one e4m3 plane:
-        1.65 times the throughput, states equal to the 8-row path's only to FP8 rounding)."""
+        states equal to the 8-row path's only to FP8 rounding; no faster where the experts' weights are the bound)."""
         if self.max_rows < min(chunk, len(ids)) and len(ids) > 1:
             chunk = self.max_rows
         ids = list(int(t) for t in ids)
